@@ -161,7 +161,7 @@ moe_combine_kernel(const __nv_bfloat16* __restrict__ ys, int d, int T, int k, co
   for (int j = 0; j < k; ++j) {
     const int row = row_of[(long long)tok * k + j];
     if (row < 0) continue;
-    const float w = topk_w[(long long)tok * k + j];
+    const float w = topk_w ? topk_w[(long long)tok * k + j] : 1.f;
     const uint4 u = *reinterpret_cast<const uint4*>(ys + (long long)row * d + c);
     const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), cc = unpack_bf16x2(u.z), dd = unpack_bf16x2(u.w);
     acc[0] += w * a.x; acc[1] += w * a.y; acc[2] += w * b.x; acc[3] += w * b.y;
@@ -175,6 +175,16 @@ moe_combine_kernel(const __nv_bfloat16* __restrict__ ys, int d, int T, int k, co
   uint4 o;
   o.x = pack_bf16x2(acc[0], acc[1]); o.y = pack_bf16x2(acc[2], acc[3]); o.z = pack_bf16x2(acc[4], acc[5]); o.w = pack_bf16x2(acc[6], acc[7]);
   *reinterpret_cast<uint4*>(out + (long long)tok * ld_out + c) = o;
+}
+
+// topk_w == nullptr: the plain sum of the rows
+int moe_combine(const void* ys, int d, int T, int k, const int* row_of, const float* topk_w, const void* resid, int ld_resid, void* out, int ld_out,
+                cudaStream_t stream) {
+  const long long total = (long long)T * (d / 8), grid = (total + 255) / 256;
+  if (grid > 0x7fffffffLL) return fail(-1, "moe_combine: too large for one launch");
+  moe_combine_kernel<<<(unsigned)grid, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(ys), d, T, k, row_of, topk_w, static_cast<const __nv_bfloat16*>(resid),
+                                                        ld_resid, static_cast<__nv_bfloat16*>(out), ld_out);
+  return launch_check("moe_combine", 1);
 }
 
 }  // namespace nfn
@@ -235,12 +245,7 @@ extern "C" int nfn_moe_combine(const void* ys, int d, int T, int k, const int* r
                                int ld_resid, void* out, int ld_out, nfn_stream_t stream) {
   if (T <= 0) return 0;
   if (!ys || !row_of || !topk_w || !out || (d & 7) || (ld_out & 7) || (resid && (ld_resid & 7))) return fail(-1, "moe_combine: bad arguments");
-  const long long total = (long long)T * (d / 8), grid = (total + 255) / 256;
-  if (grid > 0x7fffffffLL) return fail(-1, "moe_combine: too large for one launch");
-  moe_combine_kernel<<<(unsigned)grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(ys), d, T, k, row_of, topk_w, static_cast<const __nv_bfloat16*>(resid), ld_resid,
-      static_cast<__nv_bfloat16*>(out), ld_out);
-  return launch_check("moe_combine", 1);
+  return moe_combine(ys, d, T, k, row_of, topk_w, resid, ld_resid, out, ld_out, static_cast<cudaStream_t>(stream));
 }
 
 // ---- expert parallelism over peer memory --------------------------------------------------------

@@ -16,7 +16,7 @@ from ctypes import c_float, c_int, c_void_p
 import torch
 
 from . import _lib
-from .gemm import gemm, gemm_grouped_k
+from .gemm import gemm
 from .infer import swiglu_forward
 
 __all__ = ["MoEWorkspace", "moe_forward", "moe_reference", "moe_experts", "moe_experts_native_ok"]
@@ -131,14 +131,32 @@ def moe_reference(x, w_router, w_gate_up, w_down, top_k: int, *, score_fn: str =
 
 
 # --------------------------------------------------------------------------- training path --
+class _ExpertsArgs(ctypes.Structure):
+    """nfn_moe_experts_args (csrc/kernels/nfn_kernels.h)."""
+    _fields_ = [(n, c_void_p) for n in ("x", "w1", "w2", "w3", "weights", "indices", "out", "work")] + \
+               [(n, c_int) for n in ("tokens", "d", "ff", "experts", "top", "capacity_rows", "save")] + \
+               [(n, c_void_p) for n in ("dout", "scratch", "dx", "dw1", "dw2", "dw3", "dweights")]
+
+
+def _dense(t: torch.Tensor) -> torch.Tensor:
+    """Contiguous and 16-byte aligned, as the kernels' wide loads and tile copies want it."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+def _experts_lib():
+    L = _lib.load()
+    L.nfn_moe_experts_work_bytes.restype = L.nfn_moe_experts_scratch_bytes.restype = ctypes.c_longlong
+    return L
+
+
 class _MoEExpertsFn(torch.autograd.Function):
     """Dropless expert FFN with gradients. Inputs in the tensor-runtime layout: x [T, d] bf16,
     w1 / w3 [E, d, h] (gate / up), w2 [E, h, d], routing weights [T, k] (any float dtype) and
-    indices [T, k] (int64). Forward: expert-sorted permutation -> grouped tcgen05 GEMM (gate|up)
-    -> SwiGLU -> grouped GEMM (down) -> weighted combine. Backward: the same plan drives the
-    grouped input-gradient GEMMs (the stored [E, K, N] weights are already the operand layout
-    those need); weight gradients are one TN GEMM per expert over its row segment; routing
-    weights get <expert output, upstream gradient>.
+    indices [T, k] (int64). One native call per direction (``csrc/kernels/moe_experts.cu``): a stable
+    sort of the rows by expert, grouped tcgen05 products on the weights as they are stored with
+    SwiGLU and its derivative in their epilogues, weighted combine; routing weights get
+    <expert output, upstream gradient>, the weight gradients of all experts come from grouped contractions.
 
     Reference counterparts: ``moe_swiglu_forward/backward`` (``kernels.cu:12612-12862``), which
     loop per token over its k experts with dense weights and no permutation."""
@@ -148,55 +166,37 @@ class _MoEExpertsFn(torch.autograd.Function):
         T, d = x.shape
         E, _, h = w1.shape
         k = indices.shape[-1]
-        L = _lib.load()
-        ws = MoEWorkspace(T, E, k, d, h, x.device)
-        ws.topk_idx.copy_(indices)
-        ws.topk_w.copy_(weights)
-        ws.counts.copy_(torch.bincount(indices.reshape(-1), minlength=E))
-        w_gu = torch.cat([w1.transpose(1, 2), w3.transpose(1, 2)], 1).contiguous()  # [E, 2h, d]
-        w_dn = w2.transpose(1, 2).contiguous()                                     # [E, d, h]
-        _lib.check(L.nfn_moe_plan(_p(ws.counts), c_int(E), c_int(ws.max_tiles), _p(ws.offsets), _p(ws.cursor), _p(ws.tile_expert), _p(ws.plan), _st()),
-                   "nfn_moe_plan")
-        _lib.check(L.nfn_moe_permute(_p(x), c_int(x.stride(0)), c_int(T), c_int(k), c_int(d), _p(ws.topk_idx), _p(ws.offsets), _p(ws.cursor),
-                                     c_int(ws.capacity_rows), _p(ws.xs), _p(ws.row_of), _st()), "nfn_moe_permute")
-        _grouped_gemm(ws.xs, w_gu, ws.h, ws)
-        swiglu_forward(ws.h, h, out=ws.a)
-        _grouped_gemm(ws.a, w_dn, ws.ys, ws)
+        L = _experts_lib()
+        x, d1, d2, d3 = _dense(x), _dense(w1), _dense(w2), _dense(w3)
+        wt, idx = weights.to(torch.float32).contiguous(), indices.to(torch.int64).contiguous()
+        a = _ExpertsArgs(x=x.data_ptr(), w1=d1.data_ptr(), w2=d2.data_ptr(), w3=d3.data_ptr(), weights=wt.data_ptr(), indices=idx.data_ptr(),
+                         tokens=T, d=d, ff=h, experts=E, top=k, capacity_rows=(T * k + E * 127 + 127) // 128 * 128,
+                         save=int(any(ctx.needs_input_grad)))
+        work = torch.empty(L.nfn_moe_experts_work_bytes(ctypes.byref(a)), dtype=torch.uint8, device=x.device)
         out = torch.empty(T, d, dtype=torch.bfloat16, device=x.device)
-        _lib.check(L.nfn_moe_combine(_p(ws.ys), c_int(d), c_int(T), c_int(k), _p(ws.row_of), _p(ws.topk_w), _p(None), c_int(0), _p(out),
-                                     c_int(out.stride(0)), _st()), "nfn_moe_combine")
-        ctx.ws, ctx.dims = ws, (T, d, E, h, k)
-        ctx.save_for_backward(w1, w2, w3)
-        ctx.w_dtype = weights.dtype
+        a.work, a.out = work.data_ptr(), out.data_ptr()
+        _lib.check(L.nfn_moe_experts_forward(ctypes.byref(a), _st()), "nfn_moe_experts_forward")
+        if a.save:
+            ctx.save_for_backward(w1, w2, w3, wt)
+            ctx.work, ctx.dims, ctx.w_dtype = work, (T, d, E, h, k, a.capacity_rows), weights.dtype
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        from .infer import swiglu_backward
-        w1, w2, w3 = ctx.saved_tensors
-        ws, (T, d, E, h, k) = ctx.ws, ctx.dims
-        dout = dout.contiguous()
-        rows = ws.row_of.long()                                         # [T * k] sorted row of every (token, slot)
-        # routing-weight gradient and the upstream gradient of every sorted row
-        ys_tk = ws.ys[rows].view(T, k, d)
-        d_w = torch.einsum("tkd,td->tk", ys_tk.float(), dout.float())
-        dys = torch.zeros_like(ws.ys)
-        dys[rows] = (dout[:, None, :].float() * ws.topk_w[:, :, None]).to(torch.bfloat16).view(T * k, d)
-        # input gradients through the two grouped GEMMs (weights as stored are the [E, N, K] operands)
-        da = torch.empty_like(ws.a)
-        _grouped_gemm(dys, w2.contiguous(), da, ws)                     # [cap, h] = dys @ w2[e]^T
-        dh = swiglu_backward(ws.h, da, h)                               # [cap, 2h]
-        dxs = torch.empty_like(ws.xs)
-        _grouped_gemm(dh, torch.cat([w1, w3], 2).contiguous(), dxs, ws)  # [cap, d] = dh @ [w1 | w3][e]^T
-        dx = dxs[rows].view(T, k, d).float().sum(1).to(torch.bfloat16)
-        # weight gradients of all experts: three grouped contractions over the plan's padded row segments (pad rows of xs and
-        # dys are zero, those of a and dh are finite), no host read of the counts
-        dw1, dw2, dw3 = torch.empty_like(w1), torch.empty_like(w2), torch.empty_like(w3)
-        gemm_grouped_k(ws.xs, dh[:, :h], ws.offsets, dw1)               # [E, d, h] = xs^T dh_gate
-        gemm_grouped_k(ws.xs, dh[:, h:], ws.offsets, dw3)
-        gemm_grouped_k(ws.a, dys, ws.offsets, dw2)                      # [E, h, d] = a^T dys
-        ctx.ws = None
-        return dx, dw1, dw2, dw3, d_w.to(ctx.w_dtype), None
+        w1, w2, w3, wt = ctx.saved_tensors
+        T, d, E, h, k, capacity = ctx.dims
+        L, work = _experts_lib(), ctx.work
+        dout, d1, d2, d3 = _dense(dout), _dense(w1), _dense(w2), _dense(w3)
+        dx, dweights = torch.empty_like(dout), torch.empty_like(wt)
+        dw1, dw2, dw3 = (torch.empty(w.shape, dtype=w.dtype, device=w.device) for w in (w1, w2, w3))
+        a = _ExpertsArgs(w1=d1.data_ptr(), w2=d2.data_ptr(), w3=d3.data_ptr(), weights=wt.data_ptr(), work=work.data_ptr(),
+                         tokens=T, d=d, ff=h, experts=E, top=k, capacity_rows=capacity, save=1, dout=dout.data_ptr(), dx=dx.data_ptr(),
+                         dw1=dw1.data_ptr(), dw2=dw2.data_ptr(), dw3=dw3.data_ptr(), dweights=dweights.data_ptr())
+        scratch = torch.empty(L.nfn_moe_experts_scratch_bytes(ctypes.byref(a)), dtype=torch.uint8, device=dout.device)
+        a.scratch = scratch.data_ptr()
+        _lib.check(L.nfn_moe_experts_backward(ctypes.byref(a), _st()), "nfn_moe_experts_backward")
+        ctx.work = None
+        return dx, dw1, dw2, dw3, dweights.to(ctx.w_dtype), None
 
 
 def moe_experts_native_ok(x: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, w3: torch.Tensor, indices: torch.Tensor) -> bool:

@@ -56,6 +56,7 @@ KERNELS: tuple[KernelEntry, ...] = (
     _k("convolution on a sublayer's input", "nfn_input_conv", ("bf16", "fp32"), False, "per-sequence history"),
     _k("residual streams", "nfn_stream_pass", ("bf16", "fp32"), False, "mixing matrix, expert sum, norm of the update, next norm, short convolution of single tokens, row gather"),
     _k("router logits, few rows", "nfn_router_rows", ("bf16",), False, "fp32 sums"),
+    _k("experts with gradients", "nfn_moe_experts_forward", ("bf16",), True, "stable sort of rows, SwiGLU and its derivative, weights as stored, routing-weight gradient"),
     _k("experts, few rows", "nfn_moe_rows", ("bf16", "fp32"), False, "routing, item lists, weight on the input or output, clamped gate"),
     _k("residual row pass", "nfn_row_norm", ("bf16", "fp32"), False, "embedding, branch norm + residual, next norm, row gather"),
     _k("per-layer token input gate", "nfn_side_mul", ("bf16", "fp32"), False, "GELU, embedding gather"),

@@ -67,3 +67,46 @@ def test_moe_experts_autograd_matches_torch(E, k, T):
     # the stage function takes the native path for bf16 CUDA tensors
     y = SM.grouped_swiglu_experts(got_in[0].detach(), got_in[1].detach(), got_in[2].detach(), got_in[3].detach(), wts, idx)
     assert y.dtype == torch.bfloat16 and rel(y, ref) < 0.03
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,d,h,E,k,used", [
+    (1, 64, 64, 1, 1, 1),            # one row, one expert
+    (17, 64, 192, 4, 1, 2),          # a column tile that straddles the end of the hidden width, experts without rows
+    (129, 192, 320, 8, 8, 8),        # every expert for every token, widths that fill no tile
+    (1000, 512, 256, 256, 2, 256),   # the most experts
+    (2500, 256, 1088, 3, 3, 3),      # wide tiles, a remainder of the last one
+])
+def test_moe_experts_against_64_bit(kernel_lib, T, d, h, E, k, used):
+    """Results and gradients are within a few roundings to bf16 (2^-9 each) of the 64-bit values of the same bf16 inputs: rows pass three of
+    them (gate and up, their product, the output), gradients four; 2-norms average them, so 3e-3 per rounding is a bound."""
+    from neuralfn_b200.ops.moe import moe_experts
+    g = torch.Generator(device="cuda").manual_seed(T + h)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    x, w1, w2, w3, dout = r(T, d).bfloat16(), (r(E, d, h) * 0.05).bfloat16(), (r(E, h, d) * 0.05).bfloat16(), (r(E, d, h) * 0.05).bfloat16(), r(T, d).bfloat16()
+    wt, idx = torch.softmax(r(T, used), -1).topk(k, -1)
+    got_in = [t.clone().requires_grad_(True) for t in (x, w1, w2, w3, wt)]
+    got = moe_experts(*got_in, idx)
+    grads = torch.autograd.grad(got, got_in, dout)
+    ref_in = [t.double().requires_grad_(True) for t in (x, w1, w2, w3, wt)]
+    out = torch.zeros(T, d, dtype=torch.float64, device="cuda")
+    for e in range(used):
+        rows, place = (idx == e).nonzero(as_tuple=True)
+        y = (torch.nn.functional.silu(ref_in[0][rows] @ ref_in[1][e]) * (ref_in[0][rows] @ ref_in[3][e])) @ ref_in[2][e]
+        out = out.index_add(0, rows, y * ref_in[4][rows, place][:, None])
+    want = torch.autograd.grad(out, ref_in, dout.double())
+    for name, a, b in zip(("out", "dx", "dw1", "dw2", "dw3", "dweights"), (got, *grads), (out, *want)):
+        assert float((a.double() - b).norm()) <= 0.012 * float(b.norm()) + 1e-12, name
+    again = moe_experts(*got_in, idx)
+    assert torch.equal(again, got) and all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(again, got_in, dout), grads))
+
+
+@pytest.mark.gpu
+def test_moe_experts_refuses_an_expert_that_is_not_there(kernel_lib):
+    from neuralfn_b200.ops.moe import moe_experts
+    w = torch.zeros(4, 64, 64, device="cuda", dtype=torch.bfloat16)
+    x, wt = torch.zeros(3, 64, device="cuda", dtype=torch.bfloat16), torch.ones(3, 1, device="cuda")
+    for bad in (-1, 4):
+        with pytest.raises(RuntimeError):
+            moe_experts(x, w, w, w, wt, torch.tensor([[0], [bad], [1]], device="cuda"))
+    moe_experts(x, w, w, w, wt, torch.tensor([[0], [3], [1]], device="cuda"))

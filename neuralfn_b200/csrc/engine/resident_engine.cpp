@@ -190,6 +190,7 @@ int gemm(block_engine& e, const void* a, int lda, const void* b, void* cdst, int
     }
   }
   nfn_gemm_args g{};
+  const int resident = b != e.wq_scratch ? NFN_GEMM_STATIC_B : 0;  // set_tensor waits for its copy and nothing else writes weights
   g.a = a; g.b = b; g.c = cdst;
   g.m = m; g.n = n; g.k = k;
   g.lda = lda; g.ldb = k; g.ldc = ldc;
@@ -197,7 +198,7 @@ int gemm(block_engine& e, const void* a, int lda, const void* b, void* cdst, int
   // split along K, which is what lets a decode-sized product (a handful of rows) keep every SM
   // streaming weights instead of one CTA per 128 output columns
   const bool accumulate = m <= 128 && resid && resid == cdst && ld_resid == ldc && !bias && flags == 0;
-  g.flags = flags | (bias ? NFN_EPI_BIAS : 0) | (accumulate ? NFN_EPI_ACCUM : (resid ? NFN_EPI_RESID : 0));
+  g.flags = flags | resident | (bias ? NFN_EPI_BIAS : 0) | (accumulate ? NFN_EPI_ACCUM : (resid ? NFN_EPI_RESID : 0));
   g.alpha = alpha;
   g.act_param = act_param;
   g.bias = bias;

@@ -40,6 +40,24 @@ inline int launch_check(const char* what, int n_kernels = 1) {
   return 0;
 }
 
+// Launches `kern` so that its blocks may become resident while the launch before it on the stream still runs (programmatic
+// dependent launch; stream capture keeps the edge). Such a kernel calls grid_wait() in every thread before its first
+// access to memory that queued work may write or read, and before any return: its end then implies the end of all before it.
+template <typename... P, typename... A>
+inline void launch_overlapped(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);  // an error is read by launch_check
+}
+
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 }  // namespace nfn

@@ -39,6 +39,7 @@ struct DecodeParams {
   const int* lengths;
   __nv_bfloat16* out;
   int B, Hq, Hkv, cap, splits, gtiles;
+  int chunk;               // positions per split; 0: every sequence is cut into `splits` equal parts
   const __nv_bfloat16* qw;
   const __nv_bfloat16* kw;
   int qk_norm;
@@ -367,9 +368,20 @@ decode_attention_kernel(const DecodeParams p) {
 //   O += P V    HD/8 n-tiles x 1 MMA, V rows again as 16-byte chunks, two rows interleaved
 //               into a B register with one byte-permute; the output columns are permuted
 //               the same way and un-permuted once at the end.
+// Up to eight query heads take the other orientation (positions as the 16 rows, heads as the 8 columns: S^T = K Q^T,
+// O^T = V^T P^T, the weights turned around by movmatrix), which halves the MMAs and the accumulator registers; those
+// are what leaves room for loads that run ahead.
 // About 10 warp instructions per position instead of 75; no shared memory in the main loop.
 // The four warps of a CTA take alternate steps of the CTA's position range and merge at the
 // end; splits merge through the same workspace + ticket scheme as above.
+//
+// A sequence is cut by its own length, not by the batch's: ceil(length / chunk) CTAs per head group (the rest of
+// the grid leaves at once), so that one long sequence among short ones does not set the time of the launch. What
+// bounds a short launch is its chain of dependent steps, so the first K and V rows are requested before the queries
+// are prepared, the next K rows as soon as the scores have consumed the last, and the merge of the splits works from
+// weights that are computed once, its loads independent of each other.
+// Per launch, 1 sequence of 1023, 16 query heads of 128 on 4: 16.6 -> 9.1 us; 4 of up to 2047: 22.3 -> 11.5 us; 32 of 128 - 3071, 32 heads
+// on 8: 81.6 -> 52.4 us (3.6 TB/s).
 constexpr int MMA_WARPS = 4;
 constexpr int MMA_STEP = 16;  // positions per warp step
 
@@ -383,6 +395,12 @@ __device__ __forceinline__ uint4 ldg_stream16(const void* p) {
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
+// an 8 x 8 matrix of 16-bit values, lane (r, j) holding [r][2 j, 2 j + 1], transposed
+__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t v) {
+  uint32_t d;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(v));
+  return d;
+}
 __device__ __forceinline__ uint32_t word_of(const uint4& u, int i) { return i == 0 ? u.x : (i == 1 ? u.y : (i == 2 ? u.z : u.w)); }
 
 template <int HD, bool WIDE>
@@ -392,7 +410,7 @@ constexpr size_t decode_mma_smem_bytes() {
 }
 
 template <int HD, bool WIDE>
-__global__ void __launch_bounds__(MMA_WARPS * 32, 3)
+__global__ void __launch_bounds__(MMA_WARPS * 32, WIDE && HD == 128 ? 2 : 3)
 decode_attention_mma_kernel(const DecodeParams p) {
   constexpr int ROWS = WIDE ? 16 : 8;          // query-head rows kept per CTA
   constexpr int KCH = HD / 32;                 // 16-byte chunks of a K row per lane
@@ -401,12 +419,14 @@ decode_attention_mma_kernel(const DecodeParams p) {
   constexpr int VCH = HD / 64;                 // 16-byte chunks of a V row per lane
   constexpr int CH = HD / 16, HALF = HD / 2, NPART = MMA_WARPS + 1;
   extern __shared__ __align__(128) float smem[];
-  float* sm_o = smem;                                         // [NPART][ROWS][HD]
+  float* sm_o = smem;                                         // [NPART][ROWS][HD]; later the weights of the splits [64][ROWS]
   float* sm_ml = smem + NPART * ROWS * HD;                    // [NPART][ROWS][2]
   __nv_bfloat16* sm_q = reinterpret_cast<__nv_bfloat16*>(sm_ml + NPART * ROWS * 2);  // [16][HD]
   __nv_bfloat16* sm_kn = sm_q + 16 * HD;                      // [HD] new k (rotated), then [HD] new v
   __nv_bfloat16* sm_vn = sm_kn + HD;
   __shared__ int sh_last;
+  grid_trigger();
+  grid_wait();
 
   const int split = blockIdx.x, b = blockIdx.z;
   const int kvh = blockIdx.y / p.gtiles, gt = blockIdx.y % p.gtiles;
@@ -421,6 +441,20 @@ decode_attention_mma_kernel(const DecodeParams p) {
   const int pos = len - 1;
   const int slot_new = pos % p.cap;
   const int n_slots = min(len, p.cap);
+  // this sequence's splits: `live` of them take `per` positions each
+  int live = p.splits, per;
+  if (p.chunk) {
+    per = (n_slots + min(p.splits, (n_slots + p.chunk - 1) / p.chunk) - 1) / min(p.splits, (n_slots + p.chunk - 1) / p.chunk);
+    per = (per + MMA_STEP - 1) / MMA_STEP * MMA_STEP;
+    live = (n_slots + per - 1) / per;
+    if (split >= live) return;  // uniform per CTA
+  } else {
+    per = (n_slots + live - 1) / live;
+  }
+  const int s_lo = split * per, s_hi = min(n_slots, s_lo + per);
+  const int nsteps = s_hi > s_lo ? (s_hi - s_lo + MMA_STEP - 1) / MMA_STEP : 0;
+  const int last_row = max(s_hi - 1, 0);
+
   const int tpos = min(pos, p.max_pos - 1);
   const float* cosr = p.cosT ? p.cosT + (long long)tpos * HALF : nullptr;
   const float* sinr = p.sinT ? p.sinT + (long long)tpos * HALF : nullptr;
@@ -428,6 +462,30 @@ decode_attention_mma_kernel(const DecodeParams p) {
   const __nv_bfloat16* row = p.qkv + (long long)b * p.ld;
   __nv_bfloat16* kbase = p.kc + (long long)b * p.batch_stride + (long long)kvh * p.cap * HD;
   __nv_bfloat16* vbase = p.vc + (long long)b * p.batch_stride + (long long)kvh * p.cap * HD;
+
+  // K rows s0 + r and s0 + 8 + r, V rows s0 + 2j, +1, +8, +9 of a step (clamped: masked below)
+  uint4 kq[2][KCH], vq[4][VCH];
+  auto load_k = [&](int st) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const __nv_bfloat16* kr = kbase + (long long)min(s_lo + st * MMA_STEP + 8 * h + r, last_row) * HD + j * 8;
+#pragma unroll
+      for (int c = 0; c < KCH; ++c) kq[h][c] = ldg_stream16(kr + c * 32);
+    }
+  };
+  auto load_v = [&](int st) {
+#pragma unroll
+    for (int q4 = 0; q4 < 4; ++q4) {
+      const int rr = s_lo + st * MMA_STEP + (q4 >> 1) * 8 + 2 * j + (q4 & 1);
+      const __nv_bfloat16* vr = vbase + (long long)min(rr, last_row) * HD + r * 8;
+#pragma unroll
+      for (int c = 0; c < VCH; ++c) vq[q4][c] = ldg_stream16(vr + c * 64);
+    }
+  };
+  if (warp < nsteps) {
+    load_k(warp);
+    load_v(warp);
+  }
 
   // ---- prologue: the 16 sub-groups of 8 lanes prepare one query head each (norm, rotary, scale)
   {
@@ -441,19 +499,19 @@ decode_attention_mma_kernel(const DecodeParams p) {
     }
     store_chunk<CH>(sm_q + sg * HD + sub * CH, v);
     store_chunk<CH>(sm_q + sg * HD + HALF + sub * CH, v + CH);
-    if (split == 0 && warp == 0) {  // the new token's k and v (all four sub-groups compute it, the first one stores)
+    if (split == 0 && warp == MMA_WARPS - 1) {  // the new token's k and v (all four sub-groups compute it, the first one stores)
       float kn[2 * CH], vn[2 * CH];
       load_head<HD>(row + (long long)(p.Hq + kvh) * HD, p.kw, p.qk_norm, p.eps, cosr, sinr, sign, 1.f, sub, kn);
       const __nv_bfloat16* vsrc = row + (long long)(p.Hq + p.Hkv + kvh) * HD;
       load_chunk<CH>(vsrc + sub * CH, vn);
       load_chunk<CH>(vsrc + HALF + sub * CH, vn + CH);
-      if (sg == 0) {
+      if (lane < 8) {
         store_chunk<CH>(sm_kn + sub * CH, kn);
         store_chunk<CH>(sm_kn + HALF + sub * CH, kn + CH);
         store_chunk<CH>(sm_vn + sub * CH, vn);
         store_chunk<CH>(sm_vn + HALF + sub * CH, vn + CH);
       }
-      if (sg == 0 && gt == 0) {  // exactly one CTA appends the row; nobody uses that slot's old content in this launch
+      if (lane < 8 && gt == 0) {  // exactly one CTA appends the row; nobody uses that slot's old content in this launch
         store_chunk<CH>(kbase + (long long)slot_new * HD + sub * CH, kn);
         store_chunk<CH>(kbase + (long long)slot_new * HD + HALF + sub * CH, kn + CH);
         store_chunk<CH>(vbase + (long long)slot_new * HD + sub * CH, vn);
@@ -476,124 +534,162 @@ decode_attention_mma_kernel(const DecodeParams p) {
     }
   }
 
-  float o[NT][4];
+  constexpr int OT = WIDE ? NT : NT / 2;
+  float o[OT][4];
 #pragma unroll
-  for (int t = 0; t < NT; ++t)
+  for (int t = 0; t < OT; ++t)
 #pragma unroll
     for (int i = 0; i < 4; ++i) o[t][i] = 0.f;
-  float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};  // rows r and r + 8; l is this lane's share
-
-  const int per = (n_slots + p.splits - 1) / p.splits;
-  const int s_lo = split * per, s_hi = min(n_slots, s_lo + per);
-  const int nsteps = s_hi > s_lo ? (s_hi - s_lo + MMA_STEP - 1) / MMA_STEP : 0;
-  const int last_row = max(s_hi - 1, 0);
+  float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};  // heads r, r + 8 (not WIDE: 2j, 2j + 1); l is this lane's share
 
   for (int st = warp; st < nsteps; st += MMA_WARPS) {
     const int s0 = s_lo + st * MMA_STEP;
-    // K rows s0 + r and s0 + 8 + r, V rows s0 + 2j, +1, +8, +9 (clamped: masked below)
-    uint4 kq[2][KCH], vq[4][VCH];
+    const bool more = st + MMA_WARPS < nsteps;
+    if constexpr (WIDE) {
+      // S = Q K^T for the two groups of 8 positions
+      float s[2][4];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const __nv_bfloat16* kr = kbase + (long long)min(s0 + 8 * h + r, last_row) * HD + j * 8;
+      for (int h = 0; h < 2; ++h) {
 #pragma unroll
-      for (int c = 0; c < KCH; ++c) kq[h][c] = ldg_stream16(kr + c * 32);
-    }
+        for (int i = 0; i < 4; ++i) s[h][i] = 0.f;
 #pragma unroll
-    for (int q4 = 0; q4 < 4; ++q4) {
-      const int rr = s0 + (q4 >> 1) * 8 + 2 * j + (q4 & 1);
-      const __nv_bfloat16* vr = vbase + (long long)min(rr, last_row) * HD + r * 8;
+        for (int kb = 0; kb < KB; ++kb) {
+          const int e = 2 * kb;
+          mma_bf16_16816(s[h], qa[kb], word_of(kq[h][e >> 2], e & 3), word_of(kq[h][(e + 1) >> 2], (e + 1) & 3));
+        }
+      }
+      if (more) load_k(st + MMA_WARPS);
+      // mask: columns 2j, 2j+1 of each group
 #pragma unroll
-      for (int c = 0; c < VCH; ++c) vq[q4][c] = ldg_stream16(vr + c * 64);
-    }
-    // S = Q K^T for the two groups of 8 positions
-    float s[2][4];
+      for (int h = 0; h < 2; ++h)
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+        for (int i = 0; i < 2; ++i) {
+          const int sp = s0 + 8 * h + 2 * j + i;
+          if (sp >= s_hi || sp == slot_new) { s[h][i] = -INFINITY; s[h][2 + i] = -INFINITY; }
+        }
+      // online softmax per row (rows r: elements 0,1; rows r + 8: elements 2,3)
+      uint32_t pa[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) s[h][i] = 0.f;
+      for (int hr = 0; hr < 2; ++hr) {
+        float mx = fmaxf(fmaxf(s[0][2 * hr], s[0][2 * hr + 1]), fmaxf(s[1][2 * hr], s[1][2 * hr + 1]));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        const float mn = fmaxf(m_run[hr], mx);
+        const float mu = mn == -INFINITY ? 0.f : mn;
+        const float corr = __expf(m_run[hr] - mu);
+        const float p00 = __expf(s[0][2 * hr] - mu), p01 = __expf(s[0][2 * hr + 1] - mu);
+        const float p10 = __expf(s[1][2 * hr] - mu), p11 = __expf(s[1][2 * hr + 1] - mu);
+        l_run[hr] = l_run[hr] * corr + (p00 + p01) + (p10 + p11);
+        m_run[hr] = mn;
+        pa[hr] = pack_bf16x2(p00, p01);        // a0 / a1: positions 2j, 2j+1 of the first group
+        pa[2 + hr] = pack_bf16x2(p10, p11);    // a2 / a3: of the second group
+#pragma unroll
+        for (int t = 0; t < NT; ++t) { o[t][2 * hr] *= corr; o[t][2 * hr + 1] *= corr; }
+      }
+      // O += P V: n-tile t takes element t % 8 of chunk t / 8 of this lane's V rows
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        const int c = t >> 3, x = t & 7;
+        const uint32_t sel = (x & 1) ? 0x7632u : 0x5410u;
+        const uint32_t b0 = __byte_perm(word_of(vq[0][c], x >> 1), word_of(vq[1][c], x >> 1), sel);
+        const uint32_t b1 = __byte_perm(word_of(vq[2][c], x >> 1), word_of(vq[3][c], x >> 1), sel);
+        mma_bf16_16816(o[t], pa, b0, b1);
+      }
+    } else {
+      // S^T = K Q^T: rows are the positions s0 + r, s0 + 8 + r, columns the heads
+      float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int kb = 0; kb < KB; ++kb) {
-        const int e = 2 * kb;
-        mma_bf16_16816(s[h], qa[kb], word_of(kq[h][e >> 2], e & 3), word_of(kq[h][(e + 1) >> 2], (e + 1) & 3));
+        const int c = (2 * kb) >> 2, i = (2 * kb) & 3;
+        const uint32_t ka[4] = {word_of(kq[0][c], i), word_of(kq[1][c], i), word_of(kq[0][c], i + 1), word_of(kq[1][c], i + 1)};
+        mma_bf16_16816(s, ka, qa[kb][0], qa[kb][2]);
+      }
+      if (more) load_k(st + MMA_WARPS);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int sp = s0 + 8 * h + r;
+        if (sp >= s_hi || sp == slot_new) { s[2 * h] = -INFINITY; s[2 * h + 1] = -INFINITY; }
+      }
+      // online softmax of the heads 2j, 2j + 1 over the eight lanes that share j
+      float corr[2], mu[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float mx = fmaxf(s[h], s[2 + h]);
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+        const float mn = fmaxf(m_run[h], mx);
+        mu[h] = mn == -INFINITY ? 0.f : mn;
+        corr[h] = __expf(m_run[h] - mu[h]);
+        m_run[h] = mn;
+        s[h] = __expf(s[h] - mu[h]);
+        s[2 + h] = __expf(s[2 + h] - mu[h]);
+        l_run[h] = l_run[h] * corr[h] + (s[h] + s[2 + h]);
+      }
+      const uint32_t b0 = movmatrix_trans(pack_bf16x2(s[0], s[1])), b1 = movmatrix_trans(pack_bf16x2(s[2], s[3]));
+      // O^T += V^T P^T: rows r, r + 8 of tile t are the dims 2 (t % 4), + 1 of this lane's chunk t / 4
+#pragma unroll
+      for (int t = 0; t < OT; ++t) {
+        const int c = t >> 2, w = t & 3;
+        o[t][0] *= corr[0]; o[t][1] *= corr[1]; o[t][2] *= corr[0]; o[t][3] *= corr[1];
+        const uint32_t va[4] = {__byte_perm(word_of(vq[0][c], w), word_of(vq[1][c], w), 0x5410u), __byte_perm(word_of(vq[0][c], w), word_of(vq[1][c], w), 0x7632u),
+                                __byte_perm(word_of(vq[2][c], w), word_of(vq[3][c], w), 0x5410u), __byte_perm(word_of(vq[2][c], w), word_of(vq[3][c], w), 0x7632u)};
+        mma_bf16_16816(o[t], va, b0, b1);
       }
     }
-    // mask: columns 2j, 2j+1 of each group
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int sp = s0 + 8 * h + 2 * j + i;
-        if (sp >= s_hi || sp == slot_new) { s[h][i] = -INFINITY; s[h][2 + i] = -INFINITY; }
-      }
-    // online softmax per row (rows r: elements 0,1; rows r + 8: elements 2,3)
-    uint32_t pa[4];
-#pragma unroll
-    for (int hr = 0; hr < (WIDE ? 2 : 1); ++hr) {
-      float mx = fmaxf(fmaxf(s[0][2 * hr], s[0][2 * hr + 1]), fmaxf(s[1][2 * hr], s[1][2 * hr + 1]));
-      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-      const float mn = fmaxf(m_run[hr], mx);
-      const float mu = mn == -INFINITY ? 0.f : mn;
-      const float corr = __expf(m_run[hr] - mu);
-      const float p00 = __expf(s[0][2 * hr] - mu), p01 = __expf(s[0][2 * hr + 1] - mu);
-      const float p10 = __expf(s[1][2 * hr] - mu), p11 = __expf(s[1][2 * hr + 1] - mu);
-      l_run[hr] = l_run[hr] * corr + (p00 + p01) + (p10 + p11);
-      m_run[hr] = mn;
-      pa[hr] = pack_bf16x2(p00, p01);        // a0 / a1: positions 2j, 2j+1 of the first group
-      pa[2 + hr] = pack_bf16x2(p10, p11);    // a2 / a3: of the second group
-#pragma unroll
-      for (int t = 0; t < NT; ++t) { o[t][2 * hr] *= corr; o[t][2 * hr + 1] *= corr; }
-    }
-    if (!WIDE) { pa[1] = 0u; pa[3] = 0u; }
-    // O += P V: n-tile t takes element t % 8 of chunk t / 8 of this lane's V rows
-#pragma unroll
-    for (int t = 0; t < NT; ++t) {
-      const int c = t >> 3, x = t & 7;
-      const uint32_t sel = (x & 1) ? 0x7632u : 0x5410u;
-      const uint32_t b0 = __byte_perm(word_of(vq[0][c], x >> 1), word_of(vq[1][c], x >> 1), sel);
-      const uint32_t b1 = __byte_perm(word_of(vq[2][c], x >> 1), word_of(vq[3][c], x >> 1), sel);
-      mma_bf16_16816(o[t], pa, b0, b1);
-    }
+    if (more) load_v(st + MMA_WARPS);
   }
 
   // ---- partials of this CTA: one per warp + the new token (split 0) ---------------------------
 #pragma unroll
-  for (int hr = 0; hr < (WIDE ? 2 : 1); ++hr) {
-    float l = l_run[hr];
-    l += __shfl_xor_sync(0xffffffffu, l, 1);
-    l += __shfl_xor_sync(0xffffffffu, l, 2);
-    const int rowi = r + 8 * hr;
-    if (j == 0) {
-      sm_ml[(warp * ROWS + rowi) * 2] = m_run[hr];
+  for (int h = 0; h < 2; ++h) {
+    float l = l_run[h];
+    if constexpr (WIDE) {
+      l += __shfl_xor_sync(0xffffffffu, l, 1);
+      l += __shfl_xor_sync(0xffffffffu, l, 2);
+    } else {
+      l += __shfl_xor_sync(0xffffffffu, l, 4);
+      l += __shfl_xor_sync(0xffffffffu, l, 8);
+      l += __shfl_xor_sync(0xffffffffu, l, 16);
+    }
+    const int rowi = WIDE ? r + 8 * h : 2 * j + h;
+    if (WIDE ? j == 0 : r == 0) {
+      sm_ml[(warp * ROWS + rowi) * 2] = m_run[h];
       sm_ml[(warp * ROWS + rowi) * 2 + 1] = l;
     }
+    float* orow = sm_o + (warp * ROWS + rowi) * HD;
 #pragma unroll
-    for (int t = 0; t < NT; ++t) {
-      const int d0 = (t >> 3) * 64 + (2 * j) * 8 + (t & 7);
-      sm_o[(warp * ROWS + rowi) * HD + d0] = o[t][2 * hr];
-      sm_o[(warp * ROWS + rowi) * HD + d0 + 8] = o[t][2 * hr + 1];
+    for (int t = 0; t < OT; ++t) {
+      if constexpr (WIDE) {
+        const int d0 = (t >> 3) * 64 + (2 * j) * 8 + (t & 7);
+        orow[d0] = o[t][2 * h];
+        orow[d0 + 8] = o[t][2 * h + 1];
+      } else {
+        *reinterpret_cast<float2*>(orow + (t >> 2) * 64 + r * 8 + 2 * (t & 3)) = make_float2(o[t][h], o[t][2 + h]);
+      }
     }
   }
-  if (warp == 0) {  // slot MMA_WARPS: the new token (weight exp(q.k), value v), present in split 0 only
-    for (int g = 0; g < ROWS; ++g) {
-      float d = 0.f;
-      if (split == 0 && g < gcount)
-        for (int e = lane; e < HD; e += 32) d += __bfloat162float(sm_q[g * HD + e]) * __bfloat162float(sm_kn[e]);
+  // slot MMA_WARPS: the new token (weight exp(q.k), value v), present in split 0 only
+  for (int g = warp; g < gcount; g += MMA_WARPS) {
+    float d = 0.f;
+    if (split == 0)
 #pragma unroll
-      for (int sft = 16; sft > 0; sft >>= 1) d += __shfl_xor_sync(0xffffffffu, d, sft);
-      const bool live = split == 0 && g < gcount;
-      if (lane == 0) {
-        sm_ml[(MMA_WARPS * ROWS + g) * 2] = live ? d : -INFINITY;
-        sm_ml[(MMA_WARPS * ROWS + g) * 2 + 1] = live ? 1.f : 0.f;
-      }
-      for (int e = lane; e < HD; e += 32) sm_o[(MMA_WARPS * ROWS + g) * HD + e] = live ? __bfloat162float(sm_vn[e]) : 0.f;
+      for (int e = 0; e < HD; e += 32) d += __bfloat162float(sm_q[g * HD + e + lane]) * __bfloat162float(sm_kn[e + lane]);
+#pragma unroll
+    for (int sft = 16; sft > 0; sft >>= 1) d += __shfl_xor_sync(0xffffffffu, d, sft);
+    if (lane == 0) {
+      sm_ml[(MMA_WARPS * ROWS + g) * 2] = split == 0 ? d : -INFINITY;
+      sm_ml[(MMA_WARPS * ROWS + g) * 2 + 1] = split == 0 ? 1.f : 0.f;
     }
+#pragma unroll
+    for (int e = 0; e < HD; e += 32) sm_o[(MMA_WARPS * ROWS + g) * HD + e + lane] = split == 0 ? __bfloat162float(sm_vn[e + lane]) : 0.f;
   }
   __syncthreads();
   const long long unit = ((long long)b * p.Hkv + kvh) * p.gtiles + gt;
   float* po = p.part_o + (unit * p.splits + split) * (long long)(ROWS * HD);
   float* pml = p.part_ml + (unit * p.splits + split) * (long long)(ROWS * 2);
-  for (int e = threadIdx.x; e < ROWS * HD; e += blockDim.x) {
+  __nv_bfloat16* out = p.out + (long long)b * p.Hq * HD + (long long)(kvh * group + g0) * HD;
+  for (int e = threadIdx.x; e < gcount * HD; e += MMA_WARPS * 32) {
     const int g = e / HD, d = e % HD;
     float mx = -INFINITY;
 #pragma unroll
@@ -607,17 +703,22 @@ decode_attention_mma_kernel(const DecodeParams p) {
         ls += w * sm_ml[(q * ROWS + g) * 2 + 1];
       }
     }
+    if (live == 1) {
+      out[e] = __float2bfloat16(ls > 0.f ? acc / ls : 0.f);
+      continue;
+    }
     po[e] = acc;
     if (d == 0) {
       pml[g * 2] = mx;
       pml[g * 2 + 1] = ls;
     }
   }
+  if (live == 1) return;
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
     const int t = atomicAdd(&p.tickets[unit], 1);
-    sh_last = (t == p.splits - 1);
+    sh_last = (t == live - 1);
     if (sh_last) p.tickets[unit] = 0;
   }
   __syncthreads();
@@ -625,18 +726,40 @@ decode_attention_mma_kernel(const DecodeParams p) {
   __threadfence();
   const float* ao = p.part_o + unit * p.splits * (long long)(ROWS * HD);
   const float* aml = p.part_ml + unit * p.splits * (long long)(ROWS * 2);
-  for (int e = threadIdx.x; e < gcount * HD; e += blockDim.x) {
-    const int g = e / HD, d = e % HD;
-    float mx = -INFINITY;
-    for (int s = 0; s < p.splits; ++s) mx = fmaxf(mx, __ldcg(aml + (s * ROWS + g) * 2));
-    float acc = 0.f, ls = 0.f;
-    if (mx != -INFINITY)
-      for (int s = 0; s < p.splits; ++s) {
-        const float w = __expf(__ldcg(aml + (s * ROWS + g) * 2) - mx);
-        acc += w * __ldcg(ao + (long long)(s * ROWS + g) * HD + d);
-        ls += w * __ldcg(aml + (s * ROWS + g) * 2 + 1);
-      }
-    p.out[(long long)b * p.Hq * HD + (long long)(kvh * group + g0 + g) * HD + d] = __float2bfloat16(ls > 0.f ? acc / ls : 0.f);
+  // weight of every split (at most 64: two per lane), divided by the sum
+  for (int g = warp; g < gcount; g += MMA_WARPS) {
+    float m2[2], l2[2], mx = -INFINITY, ls = 0.f;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int s = lane + 32 * h;
+      m2[h] = s < live ? __ldcg(aml + (s * ROWS + g) * 2) : -INFINITY;
+      l2[h] = s < live ? __ldcg(aml + (s * ROWS + g) * 2 + 1) : 0.f;
+      mx = fmaxf(mx, m2[h]);
+    }
+#pragma unroll
+    for (int sft = 16; sft > 0; sft >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, sft));
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      m2[h] = mx == -INFINITY ? 0.f : __expf(m2[h] - mx);
+      ls += m2[h] * l2[h];
+    }
+#pragma unroll
+    for (int sft = 16; sft > 0; sft >>= 1) ls += __shfl_xor_sync(0xffffffffu, ls, sft);
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (lane + 32 * h < live) sm_o[(lane + 32 * h) * ROWS + g] = ls > 0.f ? m2[h] / ls : 0.f;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x * 4; e < gcount * HD; e += MMA_WARPS * 32 * 4) {
+    const int g = e / HD;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int s = 0; s < live; ++s) {
+      const float w = sm_o[s * ROWS + g];
+      const float4 v = __ldcg(reinterpret_cast<const float4*>(ao + (long long)s * (ROWS * HD) + e));
+      acc.x += w * v.x; acc.y += w * v.y; acc.z += w * v.z; acc.w += w * v.w;
+    }
+    *reinterpret_cast<uint2*>(out + e) = make_uint2(pack_bf16x2(acc.x, acc.y), pack_bf16x2(acc.z, acc.w));
   }
 }
 
@@ -645,7 +768,7 @@ static int launch_decode_mma(const DecodeParams& p, cudaStream_t st) {
   constexpr size_t smem = decode_mma_smem_bytes<HD, WIDE>();
   static_assert(smem <= 48 * 1024, "decode_attention_mma: static budget");
   dim3 grid(p.splits, p.Hkv * p.gtiles, p.B);
-  decode_attention_mma_kernel<HD, WIDE><<<grid, MMA_WARPS * 32, smem, st>>>(p);
+  launch_overlapped(decode_attention_mma_kernel<HD, WIDE>, grid, MMA_WARPS * 32, smem, st, p);
   return launch_check("decode_attention_mma", 1);
 }
 
@@ -712,15 +835,26 @@ extern "C" int nfn_decode_attention(const void* qkv, int ld, void* k_cache, void
   const int group = n_q_heads / n_kv_heads;
   const int G = use_mma ? (group > 8 ? 16 : 8) : (group >= 4 ? 4 : (group >= 2 ? 2 : 1)), gtiles = (group + G - 1) / G;
   const long long units = (long long)B * n_kv_heads * gtiles;
+  const long long ticket_bytes = ((units * 4 + 255) / 256) * 256;
+  const long long split_bytes = units * (long long)G * (head_dim + 2) * 4;
+  int chunk = 0;
   if (splits <= 0) {
     // one full wave at two (SIMT) or three (tensor-core kernel) resident CTAs per SM (rounding
     // down, so no straggler wave), and at least 128 cache positions per split
     const long long want = ((use_mma ? 3LL : 2LL) * sm_count()) / units;
     splits = (int)std::max<long long>(1, std::min<long long>(want, (cap + 127) / 128));
+    if (use_mma) {
+      // Cut by the sequence: 64 positions (one step per warp) while the launch is a matter of latency, up to 256 (four
+      // steps) when there are many units, so that preparing the queries does not outweigh the stream. As many
+      // splits as the workspace holds, at least the number above.
+      chunk = 64;
+      while (chunk < 256 && units * ((cap + chunk - 1) / chunk) > 6LL * sm_count()) chunk *= 2;
+      const long long fit = std::min<long long>(64, (workspace_bytes - ticket_bytes) / split_bytes);
+      splits = (int)std::max<long long>(splits, std::min<long long>(fit, (cap + chunk - 1) / chunk));
+    }
   }
   splits = min(splits, 64);
-  const long long ticket_bytes = ((units * 4 + 255) / 256) * 256;
-  const long long need = ticket_bytes + units * splits * (long long)G * (head_dim + 2) * 4;
+  const long long need = ticket_bytes + splits * split_bytes;
   if (workspace_bytes < need) return fail(-1, "decode_attention: workspace too small (see nfn_decode_attention_workspace_bytes)");
   if (reinterpret_cast<uintptr_t>(workspace) % 16) return fail(-1, "decode_attention: workspace must be 16-byte aligned");
   DecodeParams p;
@@ -731,7 +865,7 @@ extern "C" int nfn_decode_attention(const void* qkv, int ld, void* k_cache, void
   p.batch_stride = cache_batch_stride;
   p.lengths = lengths;
   p.out = static_cast<__nv_bfloat16*>(out);
-  p.B = B; p.Hq = n_q_heads; p.Hkv = n_kv_heads; p.cap = cap; p.splits = splits; p.gtiles = gtiles;
+  p.B = B; p.Hq = n_q_heads; p.Hkv = n_kv_heads; p.cap = cap; p.splits = splits; p.gtiles = gtiles; p.chunk = chunk;
   p.qw = static_cast<const __nv_bfloat16*>(q_norm_weight);
   p.kw = static_cast<const __nv_bfloat16*>(k_norm_weight);
   p.qk_norm = qk_norm; p.eps = eps;

@@ -36,6 +36,7 @@ struct SkinnyParams {
   const __nv_bfloat16* resid;
   int m, n, k, lda, ldb, ldc, ld_resid, ld_copy;
   int act, accum, out_f32;
+  int static_b;           // weights may be fetched before the launch ahead of this one is complete
   float alpha, act_param;
 };
 
@@ -107,21 +108,27 @@ gemm_skinny_kernel(const SkinnyParams p) {
     arow[mt][1] = p.a + (size_t)min(mt * 16 + g + 8, p.m - 1) * p.lda + 8 * j;
   }
 
-  for (int c0 = c_lo; c0 < c_hi; c0 += SK_UNROLL) {
-    uint4 w[SK_UNROLL][SK_NT];
+  uint4 w[SK_UNROLL][SK_NT];
+  auto load = [&](int c0) {
 #pragma unroll
     for (int u = 0; u < SK_UNROLL; ++u) {
       const bool ok = c0 + u < c_hi;
 #pragma unroll
       for (int nt = 0; nt < SK_NT; ++nt) w[u][nt] = ok ? sk_ld_stream(wrow[nt] + (size_t)(c0 + u) * 32) : make_uint4(0, 0, 0, 0);
     }
+  };
+  grid_trigger();
+  if (p.static_b) load(c_lo);
+  grid_wait();
+  for (int c0 = c_lo; c0 < c_hi; c0 += SK_UNROLL) {
+    if (!p.static_b || c0 != c_lo) load(c0);
 #pragma unroll
     for (int u = 0; u < SK_UNROLL; ++u) {
       if (c0 + u >= c_hi) break;
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
-        const uint4 x0 = __ldg(reinterpret_cast<const uint4*>(arow[mt][0] + (size_t)(c0 + u) * 32));
-        const uint4 x1 = __ldg(reinterpret_cast<const uint4*>(arow[mt][1] + (size_t)(c0 + u) * 32));
+        const uint4 x0 = ld_after_wait16(arow[mt][0] + (size_t)(c0 + u) * 32);
+        const uint4 x1 = ld_after_wait16(arow[mt][1] + (size_t)(c0 + u) * 32);
 #pragma unroll
         for (int nt = 0; nt < SK_NT; ++nt) {
           sk_mma(acc[mt][nt], x0.x, x1.x, x0.y, x1.y, w[u][nt].x, w[u][nt].y);
@@ -424,6 +431,7 @@ int try_launch_skinny(const nfn_gemm_args& a, cudaStream_t stream) {
   p.act = (a.flags >> NFN_EPI_ACT_SHIFT) & 0xF;
   p.accum = (a.flags & NFN_EPI_ACCUM) ? 1 : 0;
   p.alpha = a.alpha; p.act_param = a.act_param;
+  p.static_b = (a.flags & NFN_GEMM_STATIC_B) ? 1 : 0;
   const int mt = (a.m + 15) / 16;
   // mode 3: the register-resident cluster form for every product up to 32 rows (measured slower than both other paths, see above)
   if (g_skinny_mode == 3 && mt <= 2) {
@@ -435,9 +443,9 @@ int try_launch_skinny(const nfn_gemm_args& a, cudaStream_t stream) {
   const size_t smem = (size_t)SK_WARPS * (mt <= 1 ? 16 : (mt <= 2 ? 32 : 64)) * (SK_ROWS + 1) * sizeof(float);
   cudaError_t e = cudaSuccess;
   if (mt <= 1) {
-    gemm_skinny_kernel<1><<<grid, SK_THREADS, smem, stream>>>(p);
+    launch_overlapped(gemm_skinny_kernel<1>, grid, SK_THREADS, smem, stream, p);
   } else if (mt <= 2) {
-    gemm_skinny_kernel<2><<<grid, SK_THREADS, smem, stream>>>(p);
+    launch_overlapped(gemm_skinny_kernel<2>, grid, SK_THREADS, smem, stream, p);
   } else {
     static bool raised = false;
     if (!raised) {
@@ -445,7 +453,7 @@ int try_launch_skinny(const nfn_gemm_args& a, cudaStream_t stream) {
       raised = e == cudaSuccess;
     }
     if (e != cudaSuccess) return fail(-2, "gemm_skinny: cannot raise the dynamic shared memory limit");
-    gemm_skinny_kernel<4><<<grid, SK_THREADS, smem, stream>>>(p);
+    launch_overlapped(gemm_skinny_kernel<4>, grid, SK_THREADS, smem, stream, p);
   }
   const int rc = launch_check("gemm_skinny", 1);
   return rc == 0 ? 1 : rc;

@@ -24,6 +24,7 @@ struct GemvParams {
   const __nv_bfloat16* resid;
   int n, k, lda, ldb, ldc, ld_resid, ld_copy;
   int act, accum, out_f32;
+  int static_b;           // weights may be fetched before the launch ahead of this one is complete
   float alpha, act_param;
 };
 
@@ -52,39 +53,51 @@ __device__ __forceinline__ float gemv_dot8(const uint4& w, const float (&x)[8]) 
   return w0.x * x[0] + w0.y * x[1] + w1.x * x[2] + w1.y * x[3] + w2.x * x[4] + w2.y * x[5] + w3.x * x[6] + w3.y * x[7];
 }
 
-// A warp takes PAIRS of weight rows (n, n + 1): eight independent 16-byte streaming loads per lane
-// are in flight per iteration and every chunk of the token vectors is unpacked once for both rows.
-// The host picks the number of warps so that every warp gets the same number of pairs.
-template <int M>
+// KS warps of a CTA share a PAIR of weight rows (n, n + 1), each with a part of K: eight independent 16-byte streaming loads per
+// lane are in flight per iteration and every chunk of the token vectors is unpacked once for both rows. The host picks the number of
+// CTAs so that every one gets the same number of pairs.
+// Weights of a resident model do not wait for the launch before: the first eight loads of every warp are in flight while that
+// launch still runs, and only the token vectors are read after it.
+template <int M, int KS>
 __global__ void __launch_bounds__(GEMV_THREADS, 3)
 gemv_bf16_kernel(const GemvParams p) {
-  const int lane = threadIdx.x & 31;
-  const int warp = blockIdx.x * (GEMV_THREADS / 32) + (threadIdx.x >> 5), nwarps = gridDim.x * (GEMV_THREADS / 32);
+  constexpr int WARPS = GEMV_THREADS / 32, SLOTS = WARPS / KS;        // row pairs a CTA works on at a time
+  __shared__ float part[2][WARPS][2 * M];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = warp % KS;
   const int pairs = (p.n + 1) >> 1;
-  for (int pr = warp; pr < pairs; pr += nwarps) {
-    const int n0 = 2 * pr;
-    const bool two = n0 + 1 < p.n;
-    const __nv_bfloat16* wa = p.b + (size_t)n0 * p.ldb;
-    const __nv_bfloat16* wb = two ? wa + p.ldb : wa;  // an odd last row is read twice, its second result dropped
+  // this warp's part of K, in chunks of 256
+  const int chunks = (p.k + 255) >> 8, k_lo = chunks * sub / KS * 256, k_hi = min(p.k, chunks * (sub + 1) / KS * 256);
+  uint4 va[GEMV_UNROLL], vb[GEMV_UNROLL];
+  auto load = [&](int pr, int k0) {
+    const __nv_bfloat16* wa = p.b + (size_t)(2 * pr) * p.ldb;
+    const __nv_bfloat16* wb = 2 * pr + 1 < p.n ? wa + p.ldb : wa;     // an odd last row is read twice, its second result dropped
+#pragma unroll
+    for (int u = 0; u < GEMV_UNROLL; ++u) {
+      const int k = k0 + u * 256;
+      const bool ok = k < k_hi;
+      va[u] = ok ? gemv_ld_stream(wa + k) : make_uint4(0, 0, 0, 0);
+      vb[u] = ok ? gemv_ld_stream(wb + k) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  grid_trigger();
+  int pr = blockIdx.x * SLOTS + warp / KS;
+  bool ahead = p.static_b && pr < pairs;
+  if (ahead) load(pr, k_lo + lane * 8);
+  grid_wait();
+  for (int it = 0; pr - warp / KS < pairs; ++it, pr += gridDim.x * SLOTS) {   // the same trip count in every warp of a CTA
     float acc[2][M];
 #pragma unroll
     for (int m = 0; m < M; ++m) acc[0][m] = acc[1][m] = 0.f;
-    for (int k0 = lane * 8; k0 < p.k; k0 += 256 * GEMV_UNROLL) {
-      uint4 va[GEMV_UNROLL], vb[GEMV_UNROLL];
+    for (int k0 = k_lo + lane * 8; k0 < k_hi && pr < pairs; k0 += 256 * GEMV_UNROLL) {
+      if (!ahead) load(pr, k0);
+      ahead = false;
 #pragma unroll
       for (int u = 0; u < GEMV_UNROLL; ++u) {
         const int k = k0 + u * 256;
-        const bool ok = k < p.k;
-        va[u] = ok ? gemv_ld_stream(wa + k) : make_uint4(0, 0, 0, 0);
-        vb[u] = ok ? gemv_ld_stream(wb + k) : make_uint4(0, 0, 0, 0);
-      }
-#pragma unroll
-      for (int u = 0; u < GEMV_UNROLL; ++u) {
-        const int k = k0 + u * 256;
-        if (k >= p.k) break;
+        if (k >= k_hi) break;
 #pragma unroll
         for (int m = 0; m < M; ++m) {
-          const uint4 xv = __ldg(reinterpret_cast<const uint4*>(p.a + (size_t)m * p.lda + k));
+          const uint4 xv = ld_after_wait16(p.a + (size_t)m * p.lda + k);
           const float2 x0 = unpack_bf16x2(xv.x), x1 = unpack_bf16x2(xv.y), x2 = unpack_bf16x2(xv.z), x3 = unpack_bf16x2(xv.w);
           const float x[8] = {x0.x, x0.y, x1.x, x1.y, x2.x, x2.y, x3.x, x3.y};
           acc[0][m] += gemv_dot8(va[u], x);
@@ -92,6 +105,7 @@ gemv_bf16_kernel(const GemvParams p) {
         }
       }
     }
+    ahead = false;
 #pragma unroll
     for (int r = 0; r < 2; ++r)
 #pragma unroll
@@ -99,32 +113,48 @@ gemv_bf16_kernel(const GemvParams p) {
 #pragma unroll
         for (int s = 16; s > 0; s >>= 1) acc[r][m] += __shfl_xor_sync(0xffffffffu, acc[r][m], s);
     // lane (r * M + m) finishes output (row m, column n0 + r)
-    if (lane < 2 * M) {
-      const int r = lane / M, m = lane % M, n = n0 + r;
-      float v = 0.f;
+    const int r = lane / M, m = lane % M, n = 2 * pr + r;
+    float v = 0.f;
 #pragma unroll
-      for (int rr = 0; rr < 2; ++rr)
+    for (int rr = 0; rr < 2; ++rr)
 #pragma unroll
-        for (int mm = 0; mm < M; ++mm)
-          if (rr == r && mm == m) v = acc[rr][mm];
-      if (r == 0 || two) {
-        v *= p.alpha;
-        if (p.bias) v += __bfloat162float(p.bias[n]);
-        v = gemv_act(v, p.act, p.act_param);
-        if (p.resid) v += __bfloat162float(p.resid[(size_t)m * p.ld_resid + n]);
-        if (p.out_f32) {
-          float* cp = static_cast<float*>(p.c) + (size_t)m * p.ldc + n;
-          if (p.accum) v += *cp;
-          *cp = v;
-          if (p.copy) p.copy[(size_t)m * p.ld_copy + n] = __float2bfloat16(v);
-        } else {
-          __nv_bfloat16* cp = static_cast<__nv_bfloat16*>(p.c) + (size_t)m * p.ldc + n;
-          if (p.accum) v += __bfloat162float(*cp);
-          *cp = __float2bfloat16(v);
-        }
+      for (int mm = 0; mm < M; ++mm)
+        if (rr == r && mm == m) v = acc[rr][mm];
+    if constexpr (KS > 1) {
+      if (lane < 2 * M) part[it & 1][warp][lane] = v;
+      __syncthreads();                                                // one per round: the other buffer's readers have passed the one before
+      v = 0.f;
+      if (lane < 2 * M)
+#pragma unroll
+        for (int q = 0; q < KS; ++q) v += part[it & 1][warp - sub + q][lane];
+    }
+    if (lane < 2 * M && sub == 0 && n < p.n) {
+      v *= p.alpha;
+      if (p.bias) v += __bfloat162float(p.bias[n]);
+      v = gemv_act(v, p.act, p.act_param);
+      if (p.resid) v += __bfloat162float(p.resid[(size_t)m * p.ld_resid + n]);
+      if (p.out_f32) {
+        float* cp = static_cast<float*>(p.c) + (size_t)m * p.ldc + n;
+        if (p.accum) v += *cp;
+        *cp = v;
+        if (p.copy) p.copy[(size_t)m * p.ld_copy + n] = __float2bfloat16(v);
+      } else {
+        __nv_bfloat16* cp = static_cast<__nv_bfloat16*>(p.c) + (size_t)m * p.ldc + n;
+        if (p.accum) v += __bfloat162float(*cp);
+        *cp = __float2bfloat16(v);
       }
     }
   }
+}
+
+template <int KS>
+static void launch_gemv_bf16(const GemvParams& p, int m, cudaStream_t stream) {
+  // as many CTAs as three per SM, trimmed so that every one takes the same number of row pairs
+  constexpr int SLOTS = GEMV_THREADS / 32 / KS;
+  const int items = ((p.n + 1) / 2 + SLOTS - 1) / SLOTS, resident = sm_count() * 3, rounds = (items + resident - 1) / resident;
+  const int grid = (items + rounds - 1) / rounds;
+  if (m == 1) launch_overlapped(gemv_bf16_kernel<1, KS>, grid, GEMV_THREADS, 0, stream, p);
+  else launch_overlapped(gemv_bf16_kernel<2, KS>, grid, GEMV_THREADS, 0, stream, p);
 }
 
 // Returns 1 when it launched, 0 when the product is not a GEMV case (the caller continues with the
@@ -145,14 +175,15 @@ int try_launch_gemv(const nfn_gemm_args& a, cudaStream_t stream) {
   p.act = (a.flags >> NFN_EPI_ACT_SHIFT) & 0xF;
   p.accum = (a.flags & NFN_EPI_ACCUM) ? 1 : 0;
   p.alpha = a.alpha; p.act_param = a.act_param;
-  // as many warps as three resident CTAs per SM can hold, trimmed so that every warp takes the same number of row pairs
-  const int warps_per_block = GEMV_THREADS / 32;
-  const int pairs = (a.n + 1) / 2, max_warps = sm_count() * 3 * warps_per_block;
-  const int rounds = (pairs + max_warps - 1) / max_warps;
-  const int warps = (pairs + rounds - 1) / rounds;
-  const int grid = std::max(1, (warps + warps_per_block - 1) / warps_per_block);
-  if (a.m == 1) gemv_bf16_kernel<1><<<grid, GEMV_THREADS, 0, stream>>>(p);
-  else gemv_bf16_kernel<2><<<grid, GEMV_THREADS, 0, stream>>>(p);
+  p.static_b = (a.flags & NFN_GEMM_STATIC_B) ? 1 : 0;
+  // Warps per row pair. Two where that still is one round of all resident warps: the loads of a narrow matrix are then on their way
+  // at once (3072 x 2048, one row: 4.8 us with one, 3.3 with two, 4.2 with four). Eight for long K, where one warp would come back for
+  // the next eight loads five times or more (4096 x 14336: 25.3, 25.1, 24.7, 23.1 us; two rows 35.9 and 24.5; 2048 x 5632, two rows:
+  // 12.9, 7.9, 9.4, 7.1). One otherwise: the sum over warps costs more than it gives (11264 x 2048: 10.4, 10.9, 12.9, 18.3).
+  const bool narrow = (a.n + 1) / 2 * 2 <= sm_count() * 3 * (GEMV_THREADS / 32);
+  if (a.k >= 8192 || (narrow && a.k >= 5632)) launch_gemv_bf16<8>(p, a.m, stream);
+  else if (narrow && a.k >= 512) launch_gemv_bf16<2>(p, a.m, stream);
+  else launch_gemv_bf16<1>(p, a.m, stream);
   const int rc = launch_check("gemv_bf16", 1);
   return rc == 0 ? 1 : rc;
 }

@@ -21,15 +21,17 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
 }
 
 __global__ void __launch_bounds__(256)
-swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, int ld, __nv_bfloat16* __restrict__ out, int ld_out, long long rows, int I) {
+swiglu_fwd_kernel(const __nv_bfloat16* gu, int ld, __nv_bfloat16* out, int ld_out, long long rows, int I) {
+  grid_trigger();
+  grid_wait();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int vecs = I / 8;
   if (idx >= rows * vecs) return;
   const long long r = idx / vecs;
   const int c = (int)(idx % vecs) * 8;
   float g[8], u[8], o[8];
-  unpack8(*reinterpret_cast<const uint4*>(gu + r * ld + c), g);
-  unpack8(*reinterpret_cast<const uint4*>(gu + r * ld + I + c), u);
+  unpack8(ld_after_wait16(gu + r * ld + c), g);
+  unpack8(ld_after_wait16(gu + r * ld + I + c), u);
 #pragma unroll
   for (int j = 0; j < 8; ++j) o[j] = silu_f(g[j]) * u[j];
   *reinterpret_cast<uint4*>(out + r * ld_out + c) = pack8(o);
@@ -110,7 +112,7 @@ extern "C" int nfn_swiglu_forward(const void* gate_up, int ld, void* out, int ld
     return fail(-1, "swiglu_forward: bad arguments (sizes and strides must be multiples of 8)");
   const long long total = rows * (inter / 8), grid = (total + 255) / 256;
   if (grid > 0x7fffffffLL) return fail(-1, "swiglu_forward: too large for one launch");
-  swiglu_fwd_kernel<<<(unsigned)grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_overlapped(swiglu_fwd_kernel, (unsigned)grid, 256, 0, static_cast<cudaStream_t>(stream),
       static_cast<const __nv_bfloat16*>(gate_up), ld, static_cast<__nv_bfloat16*>(out), ld_out, rows, inter);
   return launch_check("swiglu_forward", 1);
 }
@@ -191,15 +193,17 @@ namespace nfn {
 
 // att[r, c] *= sigmoid(gate[r, c])
 __global__ void __launch_bounds__(256)
-sigmoid_gate_kernel(__nv_bfloat16* __restrict__ att, int ld_att, const __nv_bfloat16* __restrict__ gate, int ld_gate, long long rows, int width) {
+sigmoid_gate_kernel(__nv_bfloat16* att, int ld_att, const __nv_bfloat16* gate, int ld_gate, long long rows, int width) {
+  grid_trigger();
+  grid_wait();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int vecs = width / 8;
   if (idx >= rows * vecs) return;
   const long long r = idx / vecs;
   const int c = (int)(idx % vecs) * 8;
   float a[8], g[8];
-  unpack8(*reinterpret_cast<const uint4*>(att + r * ld_att + c), a);
-  unpack8(*reinterpret_cast<const uint4*>(gate + r * ld_gate + c), g);
+  unpack8(ld_after_wait16(att + r * ld_att + c), a);
+  unpack8(ld_after_wait16(gate + r * ld_gate + c), g);
 #pragma unroll
   for (int j = 0; j < 8; ++j) a[j] *= 1.f / (1.f + __expf(-g[j]));
   *reinterpret_cast<uint4*>(att + r * ld_att + c) = pack8(a);
@@ -207,15 +211,17 @@ sigmoid_gate_kernel(__nv_bfloat16* __restrict__ att, int ld_att, const __nv_bflo
 
 // out[r, :] = resid[r, :] + RMS(x[r, :]) * (centered ? 1 + w : w); one 256-thread block per row
 __global__ void __launch_bounds__(256)
-rmsnorm_residual_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ resid,
-                        __nv_bfloat16* __restrict__ out, int C, float eps, int centered) {
+rmsnorm_residual_kernel(const __nv_bfloat16* x, const __nv_bfloat16* w, const __nv_bfloat16* resid,
+                        __nv_bfloat16* out, int C, float eps, int centered) {
+  grid_trigger();
+  grid_wait();
   __shared__ float red[8];
   const long long r = blockIdx.x;
   const int vecs = C / 8;
   float ss = 0.f;
   for (int v = threadIdx.x; v < vecs; v += blockDim.x) {
     float f[8];
-    unpack8(*reinterpret_cast<const uint4*>(x + r * C + v * 8), f);
+    unpack8(ld_after_wait16(x + r * C + v * 8), f);
 #pragma unroll
     for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
   }
@@ -229,12 +235,12 @@ rmsnorm_residual_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
   const float rstd = rsqrtf(tot / (float)C + eps);
   for (int v = threadIdx.x; v < vecs; v += blockDim.x) {
     float f[8], wv[8], rv[8];
-    unpack8(*reinterpret_cast<const uint4*>(x + r * C + v * 8), f);
-    unpack8(*reinterpret_cast<const uint4*>(w + v * 8), wv);
+    unpack8(ld_after_wait16(x + r * C + v * 8), f);
+    unpack8(ld_after_wait16(w + v * 8), wv);
 #pragma unroll
     for (int j = 0; j < 8; ++j) f[j] = f[j] * rstd * (centered ? 1.f + wv[j] : wv[j]);
     if (resid) {
-      unpack8(*reinterpret_cast<const uint4*>(resid + r * C + v * 8), rv);
+      unpack8(ld_after_wait16(resid + r * C + v * 8), rv);
 #pragma unroll
       for (int j = 0; j < 8; ++j) f[j] += rv[j];
     }
@@ -250,7 +256,7 @@ extern "C" int nfn_sigmoid_gate_inplace(void* att, int ld_att, const void* gate,
   if (!att || !gate || width <= 0 || (width & 7) || (ld_att & 7) || (ld_gate & 7)) return fail(-1, "sigmoid_gate: bad arguments");
   const long long total = rows * (width / 8), grid = (total + 255) / 256;
   if (grid > 0x7fffffffLL) return fail(-1, "sigmoid_gate: too large for one launch");
-  sigmoid_gate_kernel<<<(unsigned)grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<__nv_bfloat16*>(att), ld_att,
+  launch_overlapped(sigmoid_gate_kernel, (unsigned)grid, 256, 0, static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(att), ld_att,
                                                                                     static_cast<const __nv_bfloat16*>(gate), ld_gate, rows, width);
   return launch_check("sigmoid_gate", 1);
 }
@@ -262,7 +268,7 @@ extern "C" int nfn_rmsnorm_residual(const void* x, const void* weight, const voi
   using namespace nfn;
   if (rows <= 0) return 0;
   if (!x || !weight || !out || C <= 0 || (C & 7) || rows > 0x7fffffffLL) return fail(-1, "rmsnorm_residual: bad arguments");
-  rmsnorm_residual_kernel<<<(unsigned)rows, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_overlapped(rmsnorm_residual_kernel, (unsigned)rows, 256, 0, static_cast<cudaStream_t>(stream),
       static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(weight), static_cast<const __nv_bfloat16*>(resid),
       static_cast<__nv_bfloat16*>(out), C, eps, centered);
   return launch_check("rmsnorm_residual", 1);

@@ -44,6 +44,7 @@ enum {
   NFN_EPI_ACCUM = 1 << 4,     // C += result
   NFN_EPI_OUT_F32 = 1 << 5,   // C is fp32
   NFN_EPI_COPY_BF16 = 1 << 6, // with OUT_F32: also write bf16 of the final C to aux_out (ld = ld_aux_out)
+  NFN_GEMM_STATIC_B = 1 << 7, // B is written by no work queued on the device (resident weights): it may be fetched ahead of the stream's order
   NFN_EPI_ACT_SHIFT = 8,      // activation id in bits 8..11
 };
 enum { NFN_ACT_NONE = 0, NFN_ACT_GELU_TANH = 1, NFN_ACT_GELU_ERF = 2, NFN_ACT_SILU = 3,

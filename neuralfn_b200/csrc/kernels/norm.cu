@@ -38,11 +38,12 @@ __device__ __forceinline__ float row_sum(float v, float* red) {
   return t;
 }
 
-__device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&f)[8]) {
-  const uint4 u = *reinterpret_cast<const uint4*>(p);
+__device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
   float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), c = unpack_bf16x2(u.z), d = unpack_bf16x2(u.w);
   f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
 }
+__device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&f)[8]) { unpack8(*reinterpret_cast<const uint4*>(p), f); }
+__device__ __forceinline__ void load8_after_wait(const __nv_bfloat16* p, float (&f)[8]) { unpack8(ld_after_wait16(p), f); }
 __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
   uint4 u;
   u.x = pack_bf16x2(f[0], f[1]); u.y = pack_bf16x2(f[2], f[3]);
@@ -55,11 +56,13 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
 // VEC = number of 8-element vectors per lane (C <= VEC*256).
 template <int VEC, int TPR>
 __global__ void __launch_bounds__(NORM_THREADS)
-norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
-                const __nv_bfloat16* __restrict__ b, __nv_bfloat16* __restrict__ y,
-                float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int C,
+norm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* w,
+                const __nv_bfloat16* b, __nv_bfloat16* y,
+                float* mean_out, float* rstd_out, int rows, int C,
                 float eps, int mode, int centered) {
   __shared__ float red[8];
+  grid_trigger();
+  grid_wait();
   const int lane = threadIdx.x % TPR;
   const int row = blockIdx.x * (NORM_THREADS / TPR) + threadIdx.x / TPR;
   if (TPR == 32 && row >= rows) return;  // TPR == 256: one row per block, grid == rows
@@ -70,7 +73,7 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
   for (int i = 0; i < VEC; ++i) {
     const int c = (i * TPR + lane) * 8;
     if (c < C) {
-      load8(xr + c, v[i]);
+      load8_after_wait(xr + c, v[i]);
 #pragma unroll
       for (int j = 0; j < 8; ++j) s += v[i][j];
     } else {
@@ -100,8 +103,8 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
     const int c = (i * TPR + lane) * 8;
     if (c < C) {
       float o[8], wv[8], bv[8];
-      if (w) load8(w + c, wv);
-      if (b) load8(b + c, bv);
+      if (w) load8_after_wait(w + c, wv);
+      if (b) load8_after_wait(b + c, bv);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         float n = (v[i][j] - mean) * rstd;
@@ -311,7 +314,7 @@ extern "C" int nfn_norm_forward(const void* x, const void* w, const void* b, voi
     constexpr int V = decltype(vec)::value;
     constexpr int T = decltype(tpr)::value;
     const int grid = ceil_div(rows, NORM_THREADS / T);
-    norm_fwd_kernel<V, T><<<grid, NORM_THREADS, 0, st>>>(
+    launch_overlapped(norm_fwd_kernel<V, T>, grid, NORM_THREADS, 0, st,
         (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (const __nv_bfloat16*)b,
         (__nv_bfloat16*)y, mean, rstd, rows, C, eps, mode, centered);
     return launch_check("norm_fwd");

@@ -355,6 +355,18 @@ __device__ __forceinline__ float dsilu_f(float x) {
   return s * (1.f + x * (1.f - s));
 }
 
+// Programmatic dependent launch (launch_overlapped in common.h). grid_wait: all earlier work of the stream is complete and
+// visible. grid_trigger: the next launch may start filling free SMs; in kernels that allocate TMEM only after the allocation,
+// or a block of the next launch could take the columns this one still waits for.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// 16 bytes that the launch before this one wrote: a load that stays behind grid_wait (a read-only load may be moved ahead of it)
+__device__ __forceinline__ uint4 ld_after_wait16(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);

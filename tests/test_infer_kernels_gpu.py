@@ -180,6 +180,31 @@ def test_decode_attention_append_and_attend(hd, Hq, Hkv, cap, ring, decode_impl)
     assert int(ws.buf[:256].sum()) == 0  # tickets are back to zero
 
 
+@pytest.mark.parametrize("hd,Hq,Hkv,cap,B", [(128, 16, 4, 2048, 1), (64, 8, 8, 2048, 3), (128, 32, 4, 1500, 40), (64, 48, 4, 1024, 6), (128, 8, 8, 20000, 2)])
+def test_decode_attention_cut_by_length(hd, Hq, Hkv, cap, B):
+    """Lengths around the ends of a step (16), a split (64 to 256 positions) and the cache, one split and many in one launch, sequences left out."""
+    from neuralfn_b200.ops import infer
+    torch.manual_seed(Hq + cap)
+    dev = _dev()
+    edges = [1, cap, 0, 16, 17, 63, 64, 65, 128, 129, 255, 256, 257, 511, 513, cap - 1, 1025]
+    lengths = torch.tensor([cap - 37] if B == 1 else [min(edges[i % len(edges)], cap) for i in range(B)], dtype=torch.int32, device=dev)
+    kc, vc = (torch.randn(B, Hkv, cap, hd, device=dev).bfloat16() for _ in range(2))
+    qkv = torch.randn(B, (Hq + 2 * Hkv) * hd, device=dev).bfloat16()
+    ws = infer.DecodeAttentionWorkspace(B, Hq, Hkv, hd, dev)
+    x = qkv.float().view(B, Hq + 2 * Hkv, hd)
+    k_ref, v_ref = kc.clone(), vc.clone()
+    for b in range(B):
+        if int(lengths[b]):
+            k_ref[b, :, int(lengths[b]) - 1] = x[b, Hq:Hq + Hkv].bfloat16()
+            v_ref[b, :, int(lengths[b]) - 1] = x[b, Hq + Hkv:].bfloat16()
+    live = lengths > 0
+    ref = _decode_ref(x[:, :Hq], k_ref, v_ref, lengths.clamp(min=1), cap, hd ** -0.5)
+    for splits in (0, 0, 1):
+        out = infer.decode_attention(qkv, kc, vc, lengths, n_q_heads=Hq, n_kv_heads=Hkv, head_dim=hd, workspace=ws, splits=splits)
+        torch.testing.assert_close(out.float().view(B, Hq, hd)[live], ref[live], atol=2e-2, rtol=2e-2)
+    assert torch.equal(kc, k_ref) and torch.equal(vc, v_ref) and int(ws.buf[:256].sum()) == 0
+
+
 @pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K"])
 def test_kquant_dequant_matches_numpy_oracle(name):
     from neuralfn_b200.ops import infer

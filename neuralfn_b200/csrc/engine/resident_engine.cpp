@@ -182,7 +182,7 @@ int gemm(block_engine& e, const void* a, int lda, const void* b, void* cdst, int
       // a K-quant resident weight: up to eight rows with a bias / residual epilogue go to the quantised GEMV, which reads
       // the packed blocks once; everything else decodes the tensor into the scratch buffer and runs the bf16 product on it
       if (m <= 8 && flags == 0 && alpha == 1.f && (k % 256) == 0) {
-        K(nfn_kquant_gemv(it->second, b, nullptr, a, lda, cdst, ldc, bias, resid, ld_resid, m, n, k, e.stream));
+        K(nfn_kquant_gemv_resident(it->second, b, a, lda, cdst, ldc, bias, resid, ld_resid, m, n, k, e.stream));
         return 0;
       }
       K(nfn_dequant_kquant(it->second, b, (long long)n * (k / 256), e.wq_scratch, e.stream));

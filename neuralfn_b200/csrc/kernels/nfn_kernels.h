@@ -272,6 +272,9 @@ int nfn_dequant_nf4(const void* codes, const float* absmax, long long n_weights,
 // W rows are K/256 consecutive super-blocks; B <= 8.
 int nfn_kquant_gemv(int qtype, const void* w1, const void* w2, const void* x, int ldx, void* y, int ldy,
                     const void* bias, const void* resid, int ld_resid, int B, int N, int K, nfn_stream_t stream);
+// The same without a gate matrix, for weights that no work queued on the device writes: they may be fetched ahead of the stream's order.
+int nfn_kquant_gemv_resident(int qtype, const void* w, const void* x, int ldx, void* y, int ldy, const void* bias, const void* resid, int ld_resid,
+                             int B, int N, int K, nfn_stream_t stream);
 
 int nfn_allreduce_sandwich_norm(const void* const* peer_bufs, const void* multicast_buf, int* ctrl_local, int* const* ctrl_peer,
                                 int rank, int world, int epoch, const int* epoch_dev, int rows, int n, int ld, const void* bias,

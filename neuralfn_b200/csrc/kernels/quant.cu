@@ -152,6 +152,7 @@ dequant_nf4_kernel(const uint8_t* __restrict__ codes, const float* __restrict__ 
 // kilobytes are in flight per SM regardless of how few registers the math needs. The
 // activations of all batch rows sit in shared memory for the whole kernel; warp w of a stage
 // multiplies row w: every lane decodes 8 weights of each super-block from shared memory.
+constexpr size_t GEMV_SMEM_BUDGET = 200 * 1024;
 constexpr int GEMV_WARPS = 8, GEMV_STAGE_ROWS = GEMV_WARPS, GEMV_ROWS_CTA = 32;
 
 __device__ __forceinline__ void gemv_bulk_g2s(uint32_t smem_dst, const void* gsrc, uint32_t bytes, uint32_t bar) {
@@ -289,14 +290,23 @@ kquant_gemv_kernel(const uint8_t* __restrict__ W1, const uint8_t* __restrict__ W
   }
 }
 
+// The tokens and two stages of weights fit shared memory (B rounded up to 1, 2, 4 or 8 rows)
+template <class L>
+static bool gemv_fits(int B, int K, int nm) {
+  const int bt = B <= 2 ? B : (B <= 4 ? 4 : 8);
+  const size_t x_bytes = (((size_t)bt * K * 2 + 127) / 128) * 128;
+  const size_t stage = ((((size_t)GEMV_STAGE_ROWS * (K / 256) * L::kBytes) + 127) / 128) * 128 * nm;
+  return x_bytes + 2 * stage <= GEMV_SMEM_BUDGET;
+}
+
 template <class L, int BT>
 static int launch_gemv(const void* w1, const void* w2, const void* x, int ldx, void* y, int ldy, const void* bias, const void* resid,
                        int ld_resid, int B, int N, int K, cudaStream_t st) {
   const int nm = w2 ? 2 : 1;
   const size_t x_bytes = (((size_t)BT * K * 2 + 127) / 128) * 128;
   const size_t stage = ((((size_t)GEMV_STAGE_ROWS * (K / 256) * L::kBytes) + 127) / 128) * 128 * nm;
-  const size_t budget = 200 * 1024;
-  if (x_bytes + 2 * stage > budget) return fail(-1, "kquant_gemv: K too large for the shared-memory plan (split the batch or use the dequantised GEMM path)");
+  const size_t budget = GEMV_SMEM_BUDGET;
+  if (!gemv_fits<L>(BT, K, nm)) return fail(-1, "kquant_gemv: K too large for the shared-memory plan (split the batch or use the dequantised GEMM path)");
   const int n_stages = (int)std::min<size_t>(4, (budget - x_bytes) / stage);
   const size_t smem = x_bytes + (size_t)n_stages * stage;
   const dim3 grid((N + GEMV_ROWS_CTA - 1) / GEMV_ROWS_CTA);
@@ -368,9 +378,27 @@ extern "C" int nfn_dequant_nf4(const void* codes, const float* absmax, long long
   return launch_check("dequant_nf4", 1);
 }
 
+namespace nfn {
+int try_launch_gemv_q4k(const void* w, const void* x, int ldx, void* y, int ldy, const void* bias, const void* resid, int ld_resid, int b, int n, int k,
+                        bool static_w, cudaStream_t stream);  // gemv_q4k.cu
+}
+
+static int kquant_gemv(int qtype, const void* w1, const void* w2, const void* x, int ldx, void* y, int ldy, const void* bias, const void* resid, int ld_resid,
+                       int B, int N, int K, bool static_w, nfn_stream_t stream);
+
 // y[b, n] = act(W1[n, :] . x[b, :]) (* W2[n, :] . x[b, :] when w2 is given: silu-gated) + bias[n] + resid[b, n]
 extern "C" int nfn_kquant_gemv(int qtype, const void* w1, const void* w2, const void* x, int ldx, void* y, int ldy,
                                const void* bias, const void* resid, int ld_resid, int B, int N, int K, nfn_stream_t stream) {
+  return kquant_gemv(qtype, w1, w2, x, ldx, y, ldy, bias, resid, ld_resid, B, N, K, false, stream);
+}
+
+extern "C" int nfn_kquant_gemv_resident(int qtype, const void* w, const void* x, int ldx, void* y, int ldy, const void* bias, const void* resid, int ld_resid,
+                                        int B, int N, int K, nfn_stream_t stream) {
+  return kquant_gemv(qtype, w, nullptr, x, ldx, y, ldy, bias, resid, ld_resid, B, N, K, true, stream);
+}
+
+static int kquant_gemv(int qtype, const void* w1, const void* w2, const void* x, int ldx, void* y, int ldy, const void* bias, const void* resid, int ld_resid,
+                       int B, int N, int K, bool static_w, nfn_stream_t stream) {
   if (B <= 0 || N <= 0) return 0;
   if (!w1 || !x || !y) return fail(-1, "kquant_gemv: null operand");
   if (B > 8) return fail(-1, "kquant_gemv: at most 8 batch rows per call (use the dequantised GEMM path beyond)");
@@ -380,6 +408,10 @@ extern "C" int nfn_kquant_gemv(int qtype, const void* w1, const void* w2, const 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (qtype == NFN_QTYPE_Q4_K) {
     if (reinterpret_cast<uintptr_t>(w1) % 16 || reinterpret_cast<uintptr_t>(w2) % 16) return fail(-1, "kquant_gemv: weight matrices must be 16-byte aligned");
+    if (!w2 && gemv_fits<Q4KLane>(B, K, 1)) {
+      const int rc = try_launch_gemv_q4k(w1, x, ldx, y, ldy, bias, resid, ld_resid, B, N, K, static_w, st);
+      if (rc != 0) return rc < 0 ? rc : 0;
+    }
     return dispatch_gemv<Q4KLane>(w1, w2, x, ldx, y, ldy, bias, resid, ld_resid, B, N, K, st);
   }
   if (qtype == NFN_QTYPE_Q5_K) {

@@ -246,6 +246,23 @@ def test_kquant_gemv(name, B, N, K, gated):
     torch.testing.assert_close(got.float(), ref, atol=0.05 * float(ref.abs().max()), rtol=2e-2)
 
 
+@pytest.mark.parametrize("B,N,K", [(1, 16, 256), (3, 7, 512), (8, 1000, 2048 + 256), (5, 4737, 256), (1, 33, 12544), (2, 40, 13056)])
+def test_q4k_gemv_against_64_bit(B, N, K):
+    """Row tiles of 16 with a remainder, K of one super-block to the longest the tokens fit shared memory with and one beyond, more tiles than
+    CTAs. fp32 sums leave the rounding to bf16 (2^-9 of the value) and 1e-5 of the sum of magnitudes."""
+    from neuralfn_b200.ops import infer
+    from neuralfn_b200.quant import kquant
+    t, dev = kquant.GGML_TYPE["Q4_K"], _dev()
+    raw = kquant.random_blocks(t, N * K // 256, seed=N)
+    w = torch.from_numpy(kquant.dequantize(t, raw.tobytes())).view(N, K).to(dev).double()
+    x = (torch.randn(B, K, device=dev) + 0.3).bfloat16()
+    bias, resid = torch.randn(N, device=dev).bfloat16(), torch.randn(B, N, device=dev).bfloat16()
+    ref = x.double() @ w.T + bias.double() + resid.double()
+    got = infer.kquant_gemv(t, torch.from_numpy(raw).to(dev).reshape(-1), x, N, bias=bias, resid=resid)
+    bound = 2.0 ** -8 * ref.abs() + 1e-5 * (x.double().abs() @ w.abs().T)
+    assert bool(((got.double() - ref).abs() <= bound).all())
+
+
 def _block_attention_ref(qkv, kc, vc, lengths, rows, Hq, Hkv, D, window, causal, n_rows):
     """fp32 oracle: logical key list per sequence = cached positions still in the cache + block rows."""
     B, _, cap, _ = kc.shape

@@ -13,10 +13,10 @@
 //                       path as the 1-CTA kernel); the peer releases the accumulator with a
 //                       remote mbarrier arrive on the leader's barrier
 //
-// A is K-major; B is K-major (forward products X W^T) or MN-major (input gradients dY W, template
-// parameter B_MN: each CTA then stages its 128 columns of B as two 64-column panels of BK rows).
-// MN-major A, split-K and fp32 / accumulating outputs stay on the 1-CTA kernel. No load in this
-// file uses cluster multicast.
+// Either operand is K-major or MN-major (template parameters: forward products X W^T, input gradients
+// dY W, weight gradients dY^T X; an MN-major operand is staged as two 64-column panels of BK rows per
+// CTA). K may be cut into fp32 slices or into the row groups of experts. fp32 outputs other than those
+// and the residual stream stay on the 1-CTA kernel. No load in this file uses cluster multicast.
 #include <algorithm>
 
 #include "gemm_epilogue.cuh"
@@ -30,8 +30,8 @@ constexpr int P2_BM = 128;          // rows per CTA (256 per pair)
 constexpr int P2_BN = 256;          // columns per pair tile; each CTA stages 128 of the B rows
 constexpr int P2_BK = 64;
 constexpr int P2_THREADS = 320;
-constexpr int P2_STAGES = 6;
 constexpr uint32_t P2_EPI_TILE = 128 * 64 * 2;
+constexpr int P2_STAGES = 6;
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -83,7 +83,7 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
                : "memory");
 }
 
-template <bool B_MN>
+template <bool A_MN, bool B_MN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P2_THREADS, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                       const __grid_constant__ CUtensorMap tma_c, const __grid_constant__ CUtensorMap tma_aux, const GemmParams p) {
@@ -132,10 +132,17 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   cluster_sync_all();  // the peer's barriers exist before anything signals them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_trigger();
+  grid_wait();
 
   const int tiles_mn = p.tiles_m * p.tiles_n;  // pair tiles: 256 x 256
-  const int num_tiles = tiles_mn;
+  const int num_tiles = tiles_mn * p.split_k;
   const int total_kb = (p.k + BK - 1) / BK;
+  // k-blocks of slice sp: a share of K, or the rows of a group
+  auto kb_range = [&](int sp, int& lo, int& hi) {
+    lo = p.group_rows ? p.group_rows[sp] / BK : sp * p.kb_per_split;
+    hi = p.group_rows ? min(total_kb, p.group_rows[sp + 1] / BK) : min(total_kb, lo + p.kb_per_split);
+  };
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
 
   if (warp == 0) {
@@ -143,11 +150,12 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       uint32_t stage = 0, phase = 0;
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += n_pairs) {
-        int tm, tn;
-        tile_mn(p, tile, tm, tn);
+        int tm, tn, kb_lo, kb_hi;
+        tile_mn(p, tile % tiles_mn, tm, tn);
+        kb_range(tile / tiles_mn, kb_lo, kb_hi);
         const int m0 = tm * (2 * BM) + (int)rank * BM;
         const int nb0 = tn * BN + (int)rank * (BN / 2);
-        for (int kb = 0; kb < total_kb; ++kb) {
+        for (int kb = kb_lo; kb < kb_hi; ++kb) {
           if (!mbar_wait_bounded(smem_u32(&empty_bar[stage]), phase ^ 1, cta_abort, p.status, NFN_ERR_WAIT_EMPTY)) {
             ok = false;
             break;
@@ -155,7 +163,12 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
           const uint32_t fb_leader = mapa_shared(smem_u32(&full_bar[stage]), 0);
           const uint32_t sa = smem_u32(smem + stage * STAGE_BYTES);
           if (leader) mbar_expect_tx(smem_u32(&full_bar[stage]), 2 * STAGE_BYTES);
-          tma_load_2d_pair(sa, &tma_a, fb_leader, kb * BK, m0);
+          if (!A_MN) {
+            tma_load_2d_pair(sa, &tma_a, fb_leader, kb * BK, m0);
+          } else {
+#pragma unroll
+            for (int j = 0; j < BM / 64; ++j) tma_load_2d_pair(sa + j * 8192, &tma_a, fb_leader, m0 + 64 * j, kb * BK);
+          }
           if (!B_MN) {
             tma_load_2d_pair(sa + A_BYTES, &tma_b, fb_leader, kb * BK, nb0);
           } else {
@@ -168,27 +181,29 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
     }
   } else if (warp == 1) {
     if (leader && lane == 0) {
-      constexpr uint32_t idesc = make_idesc_bf16(2 * BM, BN, 0, B_MN ? 1 : 0);
+      constexpr uint32_t idesc = make_idesc_bf16(2 * BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
       uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += n_pairs) {
         if (!mbar_wait_bounded(smem_u32(&tempty_bar[acc]), acc_phase ^ 1, cta_abort, p.status, NFN_ERR_WAIT_TMEM_EMPTY)) break;
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + acc * BN;
-        for (int kb = 0; kb < total_kb; ++kb) {
+        int kb_lo, kb_hi;
+        kb_range(tile / tiles_mn, kb_lo, kb_hi);
+        for (int kb = kb_lo; kb < kb_hi; ++kb) {
           if (!mbar_wait_bounded(smem_u32(&full_bar[stage]), phase, cta_abort, p.status, NFN_ERR_WAIT_FULL)) {
             ok = false;
             break;
           }
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * STAGE_BYTES);
-          const uint64_t da = make_smem_desc_sw128(sa, 16, 1024);
+          const uint64_t da = A_MN ? make_smem_desc_sw128(sa, 8192, 1024) : make_smem_desc_sw128(sa, 16, 1024);
           const uint64_t db = B_MN ? make_smem_desc_sw128(sa + A_BYTES, 8192, 1024) : make_smem_desc_sw128(sa + A_BYTES, 16, 1024);
 #pragma unroll
           for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-            const uint64_t a_adv = (uint64_t)((UMMA_K * 2) >> 4) * kk;
-            const uint64_t b_adv = B_MN ? (uint64_t)((UMMA_K * 128) >> 4) * kk : a_adv;
-            umma_bf16_ss_pair(tmem_d, da + a_adv, db + b_adv, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+            const uint64_t a_adv = (uint64_t)((UMMA_K * (A_MN ? 128 : 2)) >> 4) * kk;
+            const uint64_t b_adv = (uint64_t)((UMMA_K * (B_MN ? 128 : 2)) >> 4) * kk;
+            umma_bf16_ss_pair(tmem_d, da + a_adv, db + b_adv, idesc, (kb > kb_lo || kk > 0) ? 1u : 0u);
           }
           umma_commit_pair(smem_u32(&empty_bar[stage]));
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -229,22 +244,19 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
 
 namespace nfn {
 
-template <bool B_MN>
-static int launch_gemm_pair(const nfn_gemm_args& a, cudaStream_t stream) {
-  constexpr size_t SMEM = 1024 + (size_t)P2_STAGES * (P2_BM * P2_BK * 2 + (P2_BN / 2) * P2_BK * 2) + 2 * P2_EPI_TILE + 256;
-  // per device: opt in to the shared-memory size once and ask how many 2-CTA clusters can be
-  // resident at the same time (GPCs with an odd number of free SMs leave one SM without a partner)
-  static int max_pairs[64] = {};
+// CTA pairs that can be resident at the same time (GPCs with an odd number of free SMs leave one SM without a partner)
+template <bool A_MN, bool B_MN>
+static int prepare_pair_kernel(size_t smem) {
+  static int max_pairs[64] = {};  // per device
   int dev = 0;
   cudaGetDevice(&dev);
-  auto kern = gemm_bf16_pair_kernel<B_MN>;
   if (!max_pairs[dev & 63]) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) != cudaSuccess)
-      return launch_check("gemm_pair attr", 0);
+    auto kern = gemm_bf16_pair_kernel<A_MN, B_MN>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return launch_check("gemm_pair attr", 0);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sm_count() & ~1, 1, 1);
     cfg.blockDim = dim3(P2_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = SMEM;
+    cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = 2;
@@ -259,19 +271,25 @@ static int launch_gemm_pair(const nfn_gemm_args& a, cudaStream_t stream) {
     }
     max_pairs[dev & 63] = std::min(n, sm_count() / 2);
   }
+  return max_pairs[dev & 63];
+}
+
+template <bool A_MN, bool B_MN>
+static int launch_pair(const nfn_gemm_args& a, int split_k, cudaStream_t stream, const int* group_rows, int groups, long long group_stride) {
+  constexpr size_t SMEM = 1024 + (size_t)P2_STAGES * (P2_BM * P2_BK * 2 + (P2_BN / 2) * P2_BK * 2) + 2 * P2_EPI_TILE + 256;
+  const int max_pairs = prepare_pair_kernel<A_MN, B_MN>(SMEM);
+  if (max_pairs <= 0) return max_pairs;
   CUtensorMap ta, tb, tc, tx;
-  if (!make_tmap_2d(&ta, a.a, 2, (uint64_t)a.k, (uint64_t)a.m, (uint64_t)a.lda, P2_BK, P2_BM, 128)) return -3;
+  if (!A_MN) {
+    if (!make_tmap_2d(&ta, a.a, 2, (uint64_t)a.k, (uint64_t)a.m, (uint64_t)a.lda, P2_BK, P2_BM, 128)) return -3;
+  } else {
+    if (!make_tmap_2d(&ta, a.a, 2, (uint64_t)a.m, (uint64_t)a.k, (uint64_t)a.lda, 64, P2_BK, 128)) return -3;
+  }
   if (!B_MN) {
     if (!make_tmap_2d(&tb, a.b, 2, (uint64_t)a.k, (uint64_t)a.n, (uint64_t)a.ldb, P2_BK, P2_BN / 2, 128)) return -3;
   } else {
     if (!make_tmap_2d(&tb, a.b, 2, (uint64_t)a.n, (uint64_t)a.k, (uint64_t)a.ldb, 64, P2_BK, 128)) return -3;
   }
-  if (a.flags & NFN_EPI_OUT_F32) tc = ta;  // fp32 outputs are stored straight from registers
-  else if (!make_tmap_2d(&tc, a.c, 2, (uint64_t)a.n, (uint64_t)a.m, (uint64_t)a.ldc, 64, P2_BM, 128)) return -3;
-  tx = tc;
-  if ((a.flags & NFN_EPI_SAVE_PRE) &&
-      !make_tmap_2d(&tx, a.aux_out, 2, (uint64_t)a.n, (uint64_t)a.m, (uint64_t)a.ld_aux_out, 64, P2_BM, 128))
-    return -3;
   GemmParams p;
   p.c = a.c;
   p.bias = static_cast<const __nv_bfloat16*>(a.bias);
@@ -282,26 +300,49 @@ static int launch_gemm_pair(const nfn_gemm_args& a, cudaStream_t stream) {
   p.flags = a.flags | epi_direct_flag(); p.alpha = a.alpha; p.act_param = a.act_param;
   p.tiles_m = ceil_div(a.m, 2 * P2_BM);
   p.tiles_n = ceil_div(a.n, P2_BN);
-  p.split_k = 1;
-  p.kb_per_split = ceil_div(a.k, P2_BK);
+  p.split_k = split_k;
+  p.kb_per_split = ceil_div(ceil_div(a.k, P2_BK), split_k);
   p.split_stride = 0;
   p.status = status_ptr();
-  p.raster_gw = pick_raster_gw(a.m, a.k, p.tiles_n);
-  const int tiles = p.tiles_m * p.tiles_n;
-  const int pairs = std::min(max_pairs[dev & 63], tiles);
-  kern<<<2 * pairs, P2_THREADS, SMEM, stream>>>(ta, tb, tc, tx, p);
+  p.raster_gw = A_MN ? 1 : pick_raster_gw(a.m, a.k, p.tiles_n);
+  tc = tx = ta;                            // fp32 outputs, slices and groups are stored straight from registers
+  if (group_rows) {
+    p.group_rows = group_rows;
+    p.split_k = groups;
+    p.split_stride = group_stride;
+    p.flags |= NFN_EPI_DIRECT_ST;
+  } else if (split_k > 1) {
+    p.split_stride = (long long)a.m * a.n;
+    p.c = a.workspace;
+    p.ldc = a.n;
+    p.flags = NFN_EPI_OUT_F32;
+    p.alpha = 1.f;
+  } else if (!(a.flags & NFN_EPI_OUT_F32)) {
+    if (!make_tmap_2d(&tc, a.c, 2, (uint64_t)a.n, (uint64_t)a.m, (uint64_t)a.ldc, 64, P2_BM, 128)) return -3;
+    tx = tc;
+    if ((a.flags & NFN_EPI_SAVE_PRE) &&
+        !make_tmap_2d(&tx, a.aux_out, 2, (uint64_t)a.n, (uint64_t)a.m, (uint64_t)a.ld_aux_out, 64, P2_BM, 128))
+      return -3;
+  }
+  const int tiles = p.tiles_m * p.tiles_n * p.split_k;
+  launch_overlapped(gemm_bf16_pair_kernel<A_MN, B_MN>, 2 * std::min(max_pairs, tiles), P2_THREADS, SMEM, stream, ta, tb, tc, tx, p);
   const int rc = launch_check("gemm_pair", 1);
   return rc < 0 ? rc : 1;
 }
 
-// Returns 1 when the problem was launched on CTA pairs, 0 when it is not eligible, < 0 on error.
-int try_launch_gemm_pair(const nfn_gemm_args& a, cudaStream_t stream) {
+// fp32 outputs go to pairs only in the residual-stream form (C += product, bf16 copy) and as split-K slices: the forms whose epilogue is
+// compiled as straight-line code.
+bool gemm_pair_ok(const nfn_gemm_args& a) {
   const bool out_f32 = a.flags & NFN_EPI_OUT_F32, accum = a.flags & NFN_EPI_ACCUM;
-  // fp32 outputs: only the residual-stream form (C += product, bf16 copy), whose epilogue is compiled as straight-line code
-  const bool residual = out_f32 && accum && (a.flags & NFN_EPI_COPY_BF16);
-  if (a.a_mn || ((out_f32 || accum) && !residual) || a.split_k > 1) return 0;
-  if (a.m < 512 || a.n < 256 || a.k < 256) return 0;
-  return a.b_mn ? launch_gemm_pair<true>(a, stream) : launch_gemm_pair<false>(a, stream);
+  return !(out_f32 || accum) || (out_f32 && accum && (a.flags & NFN_EPI_COPY_BF16));
+}
+
+// split_k > 1: fp32 slices in the workspace, summed by the caller. group_rows: see GemmParams. 1 when launched, < 0 on error.
+int launch_gemm_pair(const nfn_gemm_args& a, int split_k, cudaStream_t stream, const int* group_rows, int groups, long long group_stride) {
+  if (!a.a_mn && !a.b_mn) return launch_pair<false, false>(a, split_k, stream, group_rows, groups, group_stride);
+  if (!a.a_mn && a.b_mn) return launch_pair<false, true>(a, split_k, stream, group_rows, groups, group_stride);
+  if (a.a_mn && !a.b_mn) return launch_pair<true, false>(a, split_k, stream, group_rows, groups, group_stride);
+  return launch_pair<true, true>(a, split_k, stream, group_rows, groups, group_stride);
 }
 
 }  // namespace nfn

@@ -272,7 +272,7 @@ __device__ __forceinline__ void epi_chunk32(const GemmParams& p, uint32_t taddr,
     o[g] = pack8_bf16(v);
   }
   if (KIND == EPI_K_BIAS_GELU_SAVE) st_row32_bf16(p.aux_out + (size_t)row * p.ld_aux_out + nc, pre, wide_aux);
-  st_row32_bf16(reinterpret_cast<__nv_bfloat16*>(p.c) + (size_t)row * p.ldc + nc, o, wide_st);
+  st_row32_bf16(reinterpret_cast<__nv_bfloat16*>(p.c) + (size_t)sp * p.split_stride + (size_t)row * p.ldc + nc, o, wide_st);
 }
 
 __device__ __forceinline__ void epi_bar_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }

@@ -73,6 +73,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_trigger();
+  grid_wait();
 
   const int tiles_mn = p.tiles_m * p.tiles_n;
   const int num_tiles = tiles_mn * p.split_k;

@@ -15,8 +15,10 @@ namespace nfn {
 
 // out[m, n] = alpha * sum_s part[s][m][n] (+ out when accumulate); bf16 or fp32 output
 __global__ void __launch_bounds__(256)
-splitk_reduce_kernel(const float* __restrict__ part, long long slice, int splits, void* out, int ldc,
+splitk_reduce_kernel(const float* part, long long slice, int splits, void* out, int ldc,
                      int m, int n, float alpha, int out_f32, int accumulate, __nv_bfloat16* copy, int ld_copy) {
+  grid_trigger();
+  grid_wait();
   const int vec_per_row = n / 8;
   const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
   if (idx >= (long long)m * vec_per_row) return;
@@ -49,6 +51,14 @@ splitk_reduce_kernel(const float* __restrict__ part, long long slice, int splits
     }
     *reinterpret_cast<uint4*>(cp) = pack8_bf16(v);
   }
+}
+
+static void launch_splitk_reduce(const nfn_gemm_args& a, int split_k, cudaStream_t stream) {
+  const long long total = (long long)a.m * (a.n / 8);
+  launch_overlapped(splitk_reduce_kernel, (unsigned)((total + 255) / 256), 256, 0, stream, static_cast<const float*>(a.workspace),
+                    (long long)a.m * a.n, split_k, a.c, a.ldc, a.m, a.n, a.alpha, (a.flags & NFN_EPI_OUT_F32) ? 1 : 0,
+                    (a.flags & NFN_EPI_ACCUM) ? 1 : 0, (a.flags & NFN_EPI_COPY_BF16) ? static_cast<__nv_bfloat16*>(a.aux_out) : nullptr,
+                    a.ld_aux_out);
 }
 
 // bf16 epilogue route: 1 (default) = straight from registers with 32-byte stores, no epilogue-wide
@@ -139,21 +149,21 @@ static int launch_gemm(const nfn_gemm_args& a, int split_k, cudaStream_t stream,
   }
   const int tiles = p.tiles_m * p.tiles_n * p.split_k;
   const int grid = tiles < sm_count() ? tiles : sm_count();
-  kern<<<grid, GEMM_THREADS, SMEM, stream>>>(ta, tb, tc, tx, p);
+  launch_overlapped(kern, grid, GEMM_THREADS, SMEM, stream, ta, tb, tc, tx, p);
   int launched = 1;
   if (split_k > 1) {
-    const long long total = (long long)a.m * (a.n / 8);
-    splitk_reduce_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(
-        static_cast<const float*>(a.workspace), (long long)a.m * a.n, split_k, a.c, a.ldc, a.m, a.n,
-        a.alpha, out_f32 ? 1 : 0, accum ? 1 : 0, (a.flags & NFN_EPI_COPY_BF16) ? static_cast<__nv_bfloat16*>(a.aux_out) : nullptr, a.ld_aux_out);
+    launch_splitk_reduce(a, split_k, stream);
     launched = 2;
   }
   return launch_check("gemm", launched);
 }
 
-int try_launch_gemm_pair(const nfn_gemm_args& a, cudaStream_t stream);  // gemm_2cta.cu
 
-// CTA-pair (cta_group::2) kernel for eligible K-major products: -1 = read NFN_GEMM_PAIR once.
+// gemm_2cta.cu
+bool gemm_pair_ok(const nfn_gemm_args& a);
+int launch_gemm_pair(const nfn_gemm_args& a, int split_k, cudaStream_t stream, const int* group_rows, int groups, long long group_stride);
+
+// CTA-pair (cta_group::2) kernel: -1 = read NFN_GEMM_PAIR once.
 static int g_pair_mode = -1;
 int try_launch_gemv(const nfn_gemm_args& a, cudaStream_t stream);  // gemv_bf16.cu
 int try_launch_skinny(const nfn_gemm_args& a, cudaStream_t stream);  // gemm_skinny.cu
@@ -166,6 +176,48 @@ static bool pair_enabled() {
     g_pair_mode = (e && e[0] == '0') ? 0 : 1;  // on unless NFN_GEMM_PAIR=0
   }
   return g_pair_mode == 1;
+}
+
+// The three tile shapes of the family and what they take, in ns at full load: a k-block (64), what a tile takes beyond its k-blocks, and
+// what a launch takes beyond its tiles. A 128 x 128 or 128 x 256 tile waits for its operands (32 and 48 KB a k-block, about
+// 100 GB/s into each SM); a pair loads each half of a 256-wide B once and is bound by the tensor cores. Fitted to 43 products of 130 to
+// 50304 rows; 256 x 128 on a pair was never better than 128 x 128 and is left out.
+struct GemmTile { int bm, bn, ctas; double kb_ns, tile_ns, launch_ns; };
+constexpr GemmTile GEMM_TILES[3] = {{128, 128, 1, 330, 400, 3500}, {128, 256, 1, 460, 1000, 3500}, {256, 256, 2, 390, 1200, 4000}};
+// K slices: a second launch, and their fp32 values through L2 twice at 5 TB/s
+constexpr double GEMM_SPLIT_NS = 4500, GEMM_SPLIT_BYTES_PER_NS = 5000;
+
+struct GemmPlan { int tile, split; };
+
+// The tile shape and the number of K slices with the least estimated time. Rows x columns x K, us (start of this rule: 128 x 128 below
+// one wave of 128 x 256 tiles; pairs only above it and never for weight gradients):
+//   768 x 3072 x 16384 (gradient) 94 -> 64, 2304 x 768 x 16384 94 -> 59, 4593 x 1024 x 2816 33 -> 22, 4593 x 1024 x 1024 16 -> 12,
+//   28672 x 4096 x 8192 (gradient) 1649 -> 1474, 317 x 11264 x 2048 25 -> 20.
+static GemmPlan plan_gemm(const nfn_gemm_args& a, int sms, bool pairs, bool may_split, int fixed_split) {
+  const int kb = ceil_div(a.k, BK);
+  GemmPlan best{0, 1};
+  double best_ns = 1e300;
+  for (int t = 0; t < 3; ++t) {
+    const GemmTile& g = GEMM_TILES[t];
+    if (g.ctas == 2 && (!pairs || a.m <= 128 || a.n < 256)) continue;
+    const long long tiles = (long long)ceil_div(a.m, g.bm) * ceil_div(a.n, g.bn);
+    const int workers = sms / g.ctas;
+    for (int s = 1; s <= (may_split ? 16 : 1); ++s) {
+      const int want = fixed_split ? fixed_split : s, per = ceil_div(kb, want), split = ceil_div(kb, per);
+      if (!fixed_split && (split != s || (s > 1 && per < 8))) continue;
+      if (split > 1 && (long long)split * a.m * a.n * 4 > a.workspace_bytes) continue;
+      if (g.ctas == 2 && split == 1 && !gemm_pair_ok(a)) continue;
+      const double rounds = (double)((tiles * split + workers - 1) / workers);
+      double ns = rounds * (per * g.kb_ns + g.tile_ns) + g.launch_ns;
+      if (split > 1) ns += GEMM_SPLIT_NS + (double)split * a.m * a.n * 8 / GEMM_SPLIT_BYTES_PER_NS;
+      if (ns < best_ns) {
+        best_ns = ns;
+        best = {t, split};
+      }
+      if (fixed_split) break;
+    }
+  }
+  return best;
 }
 
 }  // namespace nfn
@@ -207,6 +259,11 @@ extern "C" int nfn_gemm_grouped_k(const nfn_gemm_args* args, const int* group_ro
   if ((reinterpret_cast<uintptr_t>(a.a) | reinterpret_cast<uintptr_t>(a.b) | reinterpret_cast<uintptr_t>(a.c)) & 15)
     return fail(-1, "gemm_grouped_k: operands must be 16-byte aligned");
   if (a.flags & ~(NFN_EPI_OUT_F32 | NFN_EPI_ACCUM)) return fail(-1, "gemm_grouped_k: only fp32 output and accumulate are supported");
+  // pairs as soon as two thirds of them have a tile: a group's K is short, so nothing else keeps the tensor cores fed
+  if (pair_enabled() && a.m > 128 && a.n >= 256 && 3ll * ceil_div(a.m, 256) * ceil_div(a.n, 256) * groups >= sm_count()) {
+    const int rc = launch_gemm_pair(a, 1, stream, group_rows, groups, group_stride);
+    return rc < 0 ? rc : 0;
+  }
   const int tiles256 = ceil_div(a.m, BM) * ceil_div(a.n, 256) * groups;
   if (tiles256 >= sm_count() && (a.n % 256 == 0 || a.n >= 1024)) return launch_gemm<256, 4, true, true>(a, 1, stream, group_rows, groups, group_stride);
   return launch_gemm<128, 6, true, true>(a, 1, stream, group_rows, groups, group_stride);
@@ -244,17 +301,16 @@ extern "C" int nfn_gemm_bf16(const nfn_gemm_args* args, nfn_stream_t stream_) {
     if (rc != 0) return rc < 0 ? rc : 0;
   }
   const int sms = sm_count();
-  const int tiles256 = ceil_div(a.m, BM) * ceil_div(a.n, 256);
-  const bool wide = tiles256 >= sms && (a.n % 256 == 0 || a.n >= 1024);
-  // split-K: only for plain products (no fused element-wise epilogue) that leave most
-  // SMs idle while K is long - the weight-gradient shapes
-  int split = 1;
+  // split-K: only for plain products (no fused element-wise epilogue)
   const int plain_mask = NFN_EPI_BIAS | NFN_EPI_SAVE_PRE | NFN_EPI_RESID | NFN_EPI_DACT | (0xF << NFN_EPI_ACT_SHIFT);
-  if (a.split_k > 1 || a.split_k == 0) {
-    const int tiles = wide ? tiles256 : ceil_div(a.m, BM) * ceil_div(a.n, 128);
-    const int kb = ceil_div(a.k, BK);
+  const bool may_split = a.split_k != 1 && !(a.flags & plain_mask) && a.workspace;
+  GemmPlan plan{0, 1};
+  if (a.m <= BM) {
+    const int tiles256 = ceil_div(a.n, 256), kb = ceil_div(a.k, BK);
+    const bool wide = tiles256 >= sms && (a.n % 256 == 0 || a.n >= 1024);
+    const int tiles = wide ? tiles256 : ceil_div(a.n, 128);
     int want = a.split_k > 1 ? a.split_k : 1;
-    if (a.split_k == 0 && a.m <= BM && kb >= 16) {
+    if (a.split_k == 0 && kb >= 16) {
       // one row tile (decode / verification: M = batch): the product only streams the weights and
       // is bound by HBM, so what matters is that every SM streams the same share. Pick the
       // k-blocks per slice that minimise waves x (slice length + per-tile overhead), with the
@@ -269,19 +325,19 @@ extern "C" int nfn_gemm_bf16(const nfn_gemm_args* args, nfn_stream_t stream_) {
         const long long cost = waves * (per + overhead_kb);
         if (best_cost < 0 || cost < best_cost) { best_cost = cost; want = s; }
       }
-    } else if (a.split_k == 0 && tiles * 2 <= sms && kb >= 32) {
-      want = sms / tiles;
-      if (want > 16) want = 16;
-      if (want > kb / 8) want = kb / 8;
     }
-    if (want > 1 && !(a.flags & plain_mask) && a.workspace &&
-        (long long)want * a.m * a.n * 4 <= a.workspace_bytes)
-      split = want;
+    plan = {wide ? 1 : 0, may_split && (long long)want * a.m * a.n * 4 <= a.workspace_bytes ? want : 1};
+  } else {
+    plan = plan_gemm(a, sms, pair_enabled(), may_split, a.split_k > 1 ? a.split_k : 0);
   }
-  if (wide && split == 1 && !a.a_mn && pair_enabled()) {
-    const int rc = try_launch_gemm_pair(a, stream);
-    if (rc != 0) return rc < 0 ? rc : 0;
+  if (plan.tile == 2) {
+    const int rc = launch_gemm_pair(a, plan.split, stream, nullptr, 0, 0);
+    if (rc < 0 || plan.split == 1) return rc < 0 ? rc : 0;
+    launch_splitk_reduce(a, plan.split, stream);
+    return launch_check("gemm", 1);
   }
+  const bool wide = plan.tile == 1;
+  const int split = plan.split;
 #define NFN_DISPATCH(AMN, BMN)                                              \
   return wide ? launch_gemm<256, 4, AMN, BMN>(a, split, stream)             \
               : launch_gemm<128, 6, AMN, BMN>(a, split, stream)

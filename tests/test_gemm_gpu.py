@@ -308,3 +308,21 @@ def test_grouped_contraction_gives_every_experts_weight_gradient(kernel_lib, m, 
     gemm_grouped_k(a, wide[:, n:], group_rows, out2)
     assert torch.equal(out2, keep)
     _lib.assert_status_ok("grouped contraction")
+
+
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
+@pytest.mark.parametrize("m,n,k,split", [(2056, 2312, 72, 1), (6664, 776, 1000, 1), (264, 520, 4104, 5), (776, 264, 16392, 0), (136, 19208, 520, 1)])
+def test_gemm_pairs_and_slices_at_edges(kernel_lib, a_mn, b_mn, m, n, k, split):
+    """Remainders of the 256 x 256 pair tile and of the k-block, an uneven last slice, in all four operand layouts; equal results on every run."""
+    from neuralfn_b200.ops import _lib
+    from neuralfn_b200.ops.gemm import gemm
+    torch.manual_seed(m)
+    a = torch.randn((k, m) if a_mn else (m, k), device="cuda", dtype=torch.bfloat16)
+    b = torch.randn((k, n) if b_mn else (n, k), device="cuda", dtype=torch.bfloat16)
+    ws = torch.empty(64 << 20, device="cuda", dtype=torch.uint8)
+    guard = torch.full((m + 1, n + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    out = gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=guard[:m, :n], workspace=ws, split_k=split)
+    again = gemm(a, b, a_mn=a_mn, b_mn=b_mn, workspace=ws, split_k=split)
+    _lib.assert_status_ok("gemm")
+    _close(out, _ref(a, b, a_mn, b_mn), k)
+    assert torch.equal(out, again) and bool((guard[m:] == 7).all()) and bool((guard[:, n:] == 7).all())

@@ -447,14 +447,16 @@ extern "C" int nfn_norm_backward_wb(const void* dy, const void* x, const float* 
 // through shared memory and writes one partial row [3][C]; norm_bwd2_final_kernel sums them.
 // The column sum of dx is the bias gradient of the linear layer that produced the residual
 // stream this norm reads (dx is d(residual stream)), so that layer needs no separate pass.
+// What bounds it is the bytes in flight: with two rows per SM slot and nothing requested during the reductions it took 44 us at
+// 16384 x 768 (100 MB). The operands of the next row are therefore requested before this one is reduced, and the grid is what is
+// resident at once, so that no second round of blocks starts cold and the partial rows stay few. With the sum of the partial rows, us:
+// 16384 x 768 53 -> 33, 3885 x 512 20 -> 11, 4593 x 1024 29 -> 16, 8192 x 4096 112 -> 65.
 constexpr int NB2_MAX_THREADS = 1024;
 
 template <bool LAYER, int MAXT>
-__global__ void __launch_bounds__(MAXT)
-norm_bwd2_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                 const __nv_bfloat16* __restrict__ w, const float* __restrict__ mean_in,
-                 const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dresid,
-                 __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int rows, int C, int tpr, int rpb,
+__global__ void __launch_bounds__(MAXT, MAXT == 384 ? 2 : 1)
+norm_bwd2_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* w, const float* mean_in,
+                 const float* rstd_in, const __nv_bfloat16* dresid, __nv_bfloat16* dx, float* partial, int rows, int C, int tpr, int rpb,
                  int centered) {
   extern __shared__ float nb2_smem[];       // [rpb][tpr * 8] column fold buffer, then [2][rpb][wpr][2] row sums
   const int wpr = tpr >> 5;
@@ -464,36 +466,48 @@ norm_bwd2_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __re
   const int lane = threadIdx.x & 31, wir = tir >> 5;
   const int c = tir * 8;
   const bool col_ok = c < C;
+  grid_trigger();
+  grid_wait();
   float wv[8], aw[8], ab[8], ac[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) { wv[j] = 1.f; aw[j] = 0.f; ab[j] = 0.f; ac[j] = 0.f; }
   if (w && col_ok) {
-    load8(w + c, wv);
+    load8_after_wait(w + c, wv);
     if (centered) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) wv[j] += 1.f;
     }
   }
   const float inv_c = 1.f / (float)C;
+  struct Row { uint4 dy, x, dresid; float mean, rstd; } next;
+  auto fetch = [&](int row) {
+    next.dy = next.x = next.dresid = make_uint4(0u, 0u, 0u, 0u);
+    next.mean = next.rstd = 0.f;
+    if (row < rows && col_ok) {
+      const size_t off = (size_t)row * C + c;
+      next.dy = ld_after_wait16(dy + off);
+      next.x = ld_after_wait16(x + off);
+      if (dresid) next.dresid = ld_after_wait16(dresid + off);
+      next.mean = LAYER ? mean_in[row] : 0.f;
+      next.rstd = rstd_in[row];
+    }
+  };
+  const int step = gridDim.x * rpb;
+  constexpr bool AHEAD = MAXT <= 512;       // 1024 threads leave 64 registers each
+  if (AHEAD) fetch(blockIdx.x * rpb + rslot);
   int it = 0;
-  for (int base = blockIdx.x * rpb; base < rows; base += gridDim.x * rpb, ++it) {
+  for (int base = blockIdx.x * rpb; base < rows; base += step, ++it) {
     const int row = base + rslot;
     const bool live = row < rows && col_ok;
-    const size_t off = (size_t)row * C + c;
-    float g[8], n[8], r[8];
-    float mean = 0.f, rstd = 0.f;
+    if (!AHEAD) fetch(row);
+    const Row cur = next;
+    if (AHEAD) fetch(row + step);
+    const float rstd = cur.rstd;
+    float g[8], n[8];
+    unpack8(cur.dy, g);
+    unpack8(cur.x, n);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) { g[j] = 0.f; n[j] = 0.f; r[j] = 0.f; }
-    if (live) {
-      float xv[8];
-      load8(dy + off, g);
-      load8(x + off, xv);
-      if (dresid) load8(dresid + off, r);
-      mean = LAYER ? mean_in[row] : 0.f;
-      rstd = rstd_in[row];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) n[j] = (xv[j] - mean) * rstd;
-    }
+    for (int j = 0; j < 8; ++j) n[j] = (n[j] - cur.mean) * rstd;
     float sg = 0.f, sgn = 0.f;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -503,7 +517,7 @@ norm_bwd2_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __re
       sg += g[j];
       sgn += g[j] * n[j];
     }
-    sg = warp_sum(sg);
+    if (LAYER) sg = warp_sum(sg);
     sgn = warp_sum(sgn);
     if (wpr > 1) {
       float* slot = s_red + ((size_t)((it & 1) * rpb + rslot) * wpr) * 2;
@@ -517,13 +531,14 @@ norm_bwd2_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __re
     sg = LAYER ? sg * inv_c : 0.f;
     sgn *= inv_c;
     if (live) {
-      float o[8];
+      float o[8], r[8];
+      unpack8(cur.dresid, r);
 #pragma unroll
       for (int j = 0; j < 8; ++j) o[j] = rstd * (g[j] - sg - n[j] * sgn) + r[j];
       uint4 u;
       u.x = pack_bf16x2(o[0], o[1]); u.y = pack_bf16x2(o[2], o[3]);
       u.z = pack_bf16x2(o[4], o[5]); u.w = pack_bf16x2(o[6], o[7]);
-      *reinterpret_cast<uint4*>(dx + off) = u;
+      *reinterpret_cast<uint4*>(dx + (size_t)row * C + c) = u;
       // sum what was stored (bf16-rounded), so the result equals a column sum of dx itself
       const float2 q0 = unpack_bf16x2(u.x), q1 = unpack_bf16x2(u.y), q2 = unpack_bf16x2(u.z), q3 = unpack_bf16x2(u.w);
       ac[0] += q0.x; ac[1] += q0.y; ac[2] += q1.x; ac[3] += q1.y;
@@ -548,9 +563,11 @@ norm_bwd2_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __re
 // Sums the partial rows [nblk][3][C]: 32 columns per block, 32 row groups per block (the loads
 // of one thread are independent, so with few hundred partial rows the chain per thread is short).
 __global__ void __launch_bounds__(1024)
-norm_bwd2_final_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ dw, __nv_bfloat16* __restrict__ db,
-                       __nv_bfloat16* __restrict__ dcol, int nblk, int C, int accumulate) {
+norm_bwd2_final_kernel(const float* partial, __nv_bfloat16* dw, __nv_bfloat16* db,
+                       __nv_bfloat16* dcol, int nblk, int C, int accumulate) {
   __shared__ float s[3][32][33];
+  grid_trigger();
+  grid_wait();
   const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
   const int col = blockIdx.x * 32 + cx;
   float a[3] = {0.f, 0.f, 0.f};
@@ -587,20 +604,27 @@ extern "C" int nfn_norm_backward_ex(const void* dy, const void* x, const void* w
   const int tpr = ((C / 8) + 31) / 32 * 32;               // threads per row, whole warps
   const int rpb = std::min(12, std::max(1, 384 / tpr));    // rows a block works on at a time (one named barrier each)
   const int threads = tpr * rpb;
-  const int per_sm = std::max(1, 1536 / threads);
-  const int grid = std::min(ceil_div(rows, rpb), std::min(per_sm * sm_count(), nfn_norm_fused_rows()));
   const size_t smem = ((size_t)rpb * tpr * 8 + (size_t)2 * rpb * (tpr / 32) * 2) * sizeof(float);
-#define NFN_NB2(L, M)                                                                                                       \
-  norm_bwd2_kernel<L, M><<<grid, threads, smem, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, mean, \
-                                                      rstd, (const __nv_bfloat16*)dresid, (__nv_bfloat16*)dx, scratch, rows, C, tpr, rpb, centered)
-  if (threads <= 512) {
-    if (mode == 0) NFN_NB2(true, 512); else NFN_NB2(false, 512);
+  int grid = 0;
+  auto run = [&](auto kern) {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem) != cudaSuccess || per_sm < 1) {
+      cudaGetLastError();
+      per_sm = 1;
+    }
+    grid = std::min(ceil_div(rows, rpb), std::min(per_sm * sm_count(), nfn_norm_fused_rows()));
+    launch_overlapped(kern, grid, threads, smem, st, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, mean, rstd,
+                      (const __nv_bfloat16*)dresid, (__nv_bfloat16*)dx, scratch, rows, C, tpr, rpb, centered);
+  };
+  if (threads <= 384) {
+    if (mode == 0) run(norm_bwd2_kernel<true, 384>); else run(norm_bwd2_kernel<false, 384>);
+  } else if (threads <= 512) {
+    if (mode == 0) run(norm_bwd2_kernel<true, 512>); else run(norm_bwd2_kernel<false, 512>);
   } else {
-    if (mode == 0) NFN_NB2(true, 1024); else NFN_NB2(false, 1024);
+    if (mode == 0) run(norm_bwd2_kernel<true, 1024>); else run(norm_bwd2_kernel<false, 1024>);
   }
-#undef NFN_NB2
-  norm_bwd2_final_kernel<<<ceil_div(C, 32), 1024, 0, st>>>(scratch, (__nv_bfloat16*)dw, (__nv_bfloat16*)db, (__nv_bfloat16*)dx_colsum, grid, C,
-                                                          accumulate);
+  launch_overlapped(norm_bwd2_final_kernel, ceil_div(C, 32), 1024, 0, st, scratch, (__nv_bfloat16*)dw, (__nv_bfloat16*)db, (__nv_bfloat16*)dx_colsum, grid, C,
+                    accumulate);
   return launch_check("norm_backward", 2);
 }
 

@@ -483,3 +483,28 @@ def test_differential_glue_kernels(kernel_lib, D):
     torch.testing.assert_close(da.float().view(N, H, 2, D), af.grad, atol=3e-3, rtol=3e-2)
     assert abs(float(dlam[0]) - float(lf.grad)) <= 2e-2 * abs(float(lf.grad)) + 1e-2
     assert dlam[1:].abs().max() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,C", [(1, 8), (3, 264), (2377, 768), (5, 1024), (700, 4096), (301, 5000), (299, 8192)])
+@pytest.mark.parametrize("mode", ["layer", "rms"])
+def test_norm_backward_rows_in_flight(kernel_lib, rows, C, mode):
+    """One row per block slot, the last one alone, all thread counts (with and without rows fetched ahead), dx over its own residual gradient.
+    dx is one rounding to bf16 of a few fp32 sums (2^-8 of the largest term); weight and bias gradients sum `rows` fp32 terms."""
+    from neuralfn_b200.ops import kernels as K
+    g = torch.Generator(device="cuda").manual_seed(rows + C)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    dy, x, dres, w = r(rows, C).bfloat16(), r(rows, C).bfloat16(), r(rows, C).bfloat16(), (1 + 0.1 * r(C)).bfloat16()
+    xd, gd = x.double(), dy.double()
+    mean = xd.mean(1) if mode == "layer" else torch.zeros(rows, device="cuda", dtype=torch.float64)
+    rstd = torch.rsqrt((xd - mean[:, None]).square().mean(1) + 1e-5)
+    n, gw = (xd - mean[:, None]) * rstd[:, None], gd * w.double()
+    want = rstd[:, None] * (gw - (gw.mean(1, keepdim=True) if mode == "layer" else 0) - n * (gw * n).mean(1, keepdim=True)) + dres.double()
+    dw, db, col = torch.empty_like(w), torch.empty_like(w), torch.empty_like(w)
+    scratch = torch.empty(K.norm_fused_rows() * 3 * C, device="cuda")
+    out = dres.clone()
+    K.norm_backward(dy, x, w, mean.float() if mode == "layer" else None, rstd.float(), dw, db, scratch, mode=K.NORM_LAYER if mode == "layer" else K.NORM_RMS,
+                    dresid=out, out=out, dx_colsum=col)
+    assert float((out.double() - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max()) + 1e-4
+    for got, ref, mag in ((dw, (gd * n).sum(0), (gd * n).abs().sum(0)), (db, gd.sum(0), gd.abs().sum(0)), (col, out.double().sum(0), out.double().abs().sum(0))):
+        assert bool(((got.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * mag + 1e-6).all())

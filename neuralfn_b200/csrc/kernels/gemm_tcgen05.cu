@@ -163,6 +163,10 @@ static int launch_gemm(const nfn_gemm_args& a, int split_k, cudaStream_t stream,
 bool gemm_pair_ok(const nfn_gemm_args& a);
 int launch_gemm_pair(const nfn_gemm_args& a, int split_k, cudaStream_t stream, const int* group_rows, int groups, long long group_stride);
 
+// gemm_slices.cu
+int launch_gemm_slices(const nfn_gemm_args& a, int slices, cudaStream_t stream);
+int gemm_slices_resident(int slices);
+
 // CTA-pair (cta_group::2) kernel: -1 = read NFN_GEMM_PAIR once.
 static int g_pair_mode = -1;
 int try_launch_gemv(const nfn_gemm_args& a, cudaStream_t stream);  // gemv_bf16.cu
@@ -178,38 +182,44 @@ static bool pair_enabled() {
   return g_pair_mode == 1;
 }
 
-// The three tile shapes of the family and what they take, in ns at full load: a k-block (64), what a tile takes beyond its k-blocks, and
+// The tile shapes of the family and what they take, in ns at full load: a k-block (64), what a tile takes beyond its k-blocks, and
 // what a launch takes beyond its tiles. A 128 x 128 or 128 x 256 tile waits for its operands (32 and 48 KB a k-block, about
-// 100 GB/s into each SM); a pair loads each half of a 256-wide B once and is bound by the tensor cores. Fitted to 43 products of 130 to
-// 50304 rows; 256 x 128 on a pair was never better than 128 x 128 and is left out.
-struct GemmTile { int bm, bn, ctas; double kb_ns, tile_ns, launch_ns; };
-constexpr GemmTile GEMM_TILES[3] = {{128, 128, 1, 330, 400, 3500}, {128, 256, 1, 460, 1000, 3500}, {256, 256, 2, 390, 1200, 4000}};
-// K slices: a second launch, and their fp32 values through L2 twice at 5 TB/s
-constexpr double GEMM_SPLIT_NS = 4500, GEMM_SPLIT_BYTES_PER_NS = 5000;
+// 100 GB/s into each SM); a pair loads each half of a 256-wide B once and is bound by the tensor cores; the last is a cluster of CTAs that
+// share one 128 x 128 tile's K. Fitted to 60 products of 32 to 50304 rows; 256 x 128 on a pair was never better than 128 x 128 and is left out.
+struct GemmTile { int bm, bn; double kb_ns, tile_ns, launch_ns; };
+enum : int { TILE_128, TILE_256, TILE_PAIR, TILE_CLUSTER };
+constexpr GemmTile GEMM_TILES[4] = {{128, 128, 330, 400, 3500}, {128, 256, 460, 1000, 3500}, {256, 256, 390, 1200, 4000}, {128, 128, 330, 400, 5600}};
+// K slices through memory: a second launch, and their fp32 values through L2 twice at 5 TB/s. Slices in a cluster: each one more rank to read.
+constexpr double GEMM_SPLIT_NS = 3500, GEMM_SPLIT_BYTES_PER_NS = 5000, GEMM_RANK_NS = 100, GEMM_HBM_BYTES_PER_NS = 5800;
 
 struct GemmPlan { int tile, split; };
 
 // The tile shape and the number of K slices with the least estimated time. Rows x columns x K, us (start of this rule: 128 x 128 below
-// one wave of 128 x 256 tiles; pairs only above it and never for weight gradients):
+// one wave of 128 x 256 tiles, slices through memory, pairs only above that wave and never for weight gradients):
 //   768 x 3072 x 16384 (gradient) 94 -> 64, 2304 x 768 x 16384 94 -> 59, 4593 x 1024 x 2816 33 -> 22, 4593 x 1024 x 1024 16 -> 12,
-//   28672 x 4096 x 8192 (gradient) 1649 -> 1474, 317 x 11264 x 2048 25 -> 20.
+//   28672 x 4096 x 8192 (gradient) 1649 -> 1474, 317 x 11264 x 2048 25 -> 20, 512 x 512 x 3885 (gradient) 13.4 -> 10.2,
+//   1024 x 256 x 2048 13.5 -> 8.3, 32 x 4096 x 14336 31.7 -> 25.5, 32 x 28672 x 4096 53.7 -> 45.5.
 static GemmPlan plan_gemm(const nfn_gemm_args& a, int sms, bool pairs, bool may_split, int fixed_split) {
   const int kb = ceil_div(a.k, BK);
-  GemmPlan best{0, 1};
+  const double stream_ns = 2.0 * ((double)a.m * a.k + (double)a.n * a.k) / GEMM_HBM_BYTES_PER_NS;
+  GemmPlan best{TILE_128, 1};
   double best_ns = 1e300;
-  for (int t = 0; t < 3; ++t) {
+  for (int t = TILE_128; t <= TILE_CLUSTER; ++t) {
     const GemmTile& g = GEMM_TILES[t];
-    if (g.ctas == 2 && (!pairs || a.m <= 128 || a.n < 256)) continue;
+    if (t == TILE_PAIR && (!pairs || a.m <= 128 || a.n < 256)) continue;
     const long long tiles = (long long)ceil_div(a.m, g.bm) * ceil_div(a.n, g.bn);
-    const int workers = sms / g.ctas;
-    for (int s = 1; s <= (may_split ? 16 : 1); ++s) {
-      const int want = fixed_split ? fixed_split : s, per = ceil_div(kb, want), split = ceil_div(kb, per);
-      if (!fixed_split && (split != s || (s > 1 && per < 8))) continue;
-      if (split > 1 && (long long)split * a.m * a.n * 4 > a.workspace_bytes) continue;
-      if (g.ctas == 2 && split == 1 && !gemm_pair_ok(a)) continue;
-      const double rounds = (double)((tiles * split + workers - 1) / workers);
-      double ns = rounds * (per * g.kb_ns + g.tile_ns) + g.launch_ns;
-      if (split > 1) ns += GEMM_SPLIT_NS + (double)split * a.m * a.n * 8 / GEMM_SPLIT_BYTES_PER_NS;
+    const bool cluster = t == TILE_CLUSTER;
+    if (cluster && (fixed_split || tiles > sms / 2)) continue;
+    for (int s = cluster ? 2 : 1; s <= (cluster ? 8 : (may_split ? 16 : 1)); ++s) {
+      const int want = fixed_split ? fixed_split : s, per = ceil_div(kb, want), split = cluster ? s : ceil_div(kb, per);
+      if (cluster ? s > kb : (!fixed_split && (split != s || (s > 1 && per < 8)))) continue;
+      if (!cluster && split > 1 && (long long)split * a.m * a.n * 4 > a.workspace_bytes) continue;
+      if (t == TILE_PAIR && split == 1 && !gemm_pair_ok(a)) continue;
+      const long long at_once = cluster ? gemm_slices_resident(s) : (t == TILE_PAIR ? sms / 2 : sms), items = cluster ? tiles : tiles * split;
+      if (at_once <= 0) continue;
+      double ns = std::max((double)((items + at_once - 1) / at_once) * (per * g.kb_ns + g.tile_ns), stream_ns) + g.launch_ns;
+      if (cluster) ns += s * GEMM_RANK_NS;
+      else if (split > 1) ns += GEMM_SPLIT_NS + (double)split * a.m * a.n * 8 / GEMM_SPLIT_BYTES_PER_NS;
       if (ns < best_ns) {
         best_ns = ns;
         best = {t, split};
@@ -304,39 +314,15 @@ extern "C" int nfn_gemm_bf16(const nfn_gemm_args* args, nfn_stream_t stream_) {
   // split-K: only for plain products (no fused element-wise epilogue)
   const int plain_mask = NFN_EPI_BIAS | NFN_EPI_SAVE_PRE | NFN_EPI_RESID | NFN_EPI_DACT | (0xF << NFN_EPI_ACT_SHIFT);
   const bool may_split = a.split_k != 1 && !(a.flags & plain_mask) && a.workspace;
-  GemmPlan plan{0, 1};
-  if (a.m <= BM) {
-    const int tiles256 = ceil_div(a.n, 256), kb = ceil_div(a.k, BK);
-    const bool wide = tiles256 >= sms && (a.n % 256 == 0 || a.n >= 1024);
-    const int tiles = wide ? tiles256 : ceil_div(a.n, 128);
-    int want = a.split_k > 1 ? a.split_k : 1;
-    if (a.split_k == 0 && kb >= 16) {
-      // one row tile (decode / verification: M = batch): the product only streams the weights and
-      // is bound by HBM, so what matters is that every SM streams the same share. Pick the
-      // k-blocks per slice that minimise waves x (slice length + per-tile overhead), with the
-      // fp32 partial slices kept below about a tenth of the weight bytes.
-      const int overhead_kb = 2;
-      const long long max_split = std::max(1LL, (long long)a.k / (20LL * a.m));
-      long long best_cost = -1;
-      for (int per = kb; per >= 2; --per) {
-        const int s = ceil_div(kb, per);
-        if (s > max_split || s > 64) break;
-        const long long waves = ((long long)tiles * s + sms - 1) / sms;
-        const long long cost = waves * (per + overhead_kb);
-        if (best_cost < 0 || cost < best_cost) { best_cost = cost; want = s; }
-      }
-    }
-    plan = {wide ? 1 : 0, may_split && (long long)want * a.m * a.n * 4 <= a.workspace_bytes ? want : 1};
-  } else {
-    plan = plan_gemm(a, sms, pair_enabled(), may_split, a.split_k > 1 ? a.split_k : 0);
-  }
-  if (plan.tile == 2) {
+  const GemmPlan plan = plan_gemm(a, sms, pair_enabled(), may_split, a.split_k > 1 ? a.split_k : 0);
+  if (plan.tile == TILE_CLUSTER) return launch_gemm_slices(a, plan.split, stream);
+  if (plan.tile == TILE_PAIR) {
     const int rc = launch_gemm_pair(a, plan.split, stream, nullptr, 0, 0);
     if (rc < 0 || plan.split == 1) return rc < 0 ? rc : 0;
     launch_splitk_reduce(a, plan.split, stream);
     return launch_check("gemm", 1);
   }
-  const bool wide = plan.tile == 1;
+  const bool wide = plan.tile == TILE_256;
   const int split = plan.split;
 #define NFN_DISPATCH(AMN, BMN)                                              \
   return wide ? launch_gemm<256, 4, AMN, BMN>(a, split, stream)             \

@@ -326,3 +326,34 @@ def test_gemm_pairs_and_slices_at_edges(kernel_lib, a_mn, b_mn, m, n, k, split):
     _lib.assert_status_ok("gemm")
     _close(out, _ref(a, b, a_mn, b_mn), k)
     assert torch.equal(out, again) and bool((guard[m:] == 7).all()) and bool((guard[:, n:] == 7).all())
+
+
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
+@pytest.mark.parametrize("m,n,k", [(136, 128, 520), (256, 264, 1032), (24, 2056, 4104), (520, 136, 6000)])
+def test_gemm_slices_in_a_cluster(kernel_lib, a_mn, b_mn, m, n, k):
+    """Fewer tiles than SMs: K cut over a cluster (uneven slices, remainders of tile and k-block, fewer rows than ranks have shares), with every epilogue."""
+    from neuralfn_b200.ops import _lib
+    from neuralfn_b200.ops.gemm import gemm
+    torch.manual_seed(m)
+    dev = "cuda"
+    a = torch.randn((k, m) if a_mn else (m, k), device=dev, dtype=torch.bfloat16)
+    b = torch.randn((k, n) if b_mn else (n, k), device=dev, dtype=torch.bfloat16)
+    bias, res = torch.randn(n, device=dev).bfloat16(), torch.randn(m, n, device=dev).bfloat16()
+    base = _ref(a, b, a_mn, b_mn)
+    guard = torch.full((m + 1, n + 8), 7.0, device=dev, dtype=torch.bfloat16)
+    _close(gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=guard[:m, :n]), base, k)
+    assert bool((guard[m:] == 7).all()) and bool((guard[:, n:] == 7).all())
+    _close(gemm(a, b, a_mn=a_mn, b_mn=b_mn, bias=bias, resid=res), base + bias.float() + res.float(), k)
+    s, pre = 1.0 / k ** 0.5, torch.empty(m, n, device=dev, dtype=torch.bfloat16)
+    y = gemm(a, b, a_mn=a_mn, b_mn=b_mn, alpha=s, act="gelu_tanh", save_pre=pre, bias=bias)
+    _close(pre, base * s + bias.float(), k)
+    _close(y, torch.nn.functional.gelu(base * s + bias.float(), approximate="tanh"), k)
+    z = res.float().requires_grad_(True)
+    torch.nn.functional.gelu(z, approximate="tanh").sum().backward()
+    _close(gemm(a, b, a_mn=a_mn, b_mn=b_mn, act="gelu_tanh", dact_pre=res), base * z.grad, k)
+    c = res.clone()
+    _close(gemm(a, b, a_mn=a_mn, b_mn=b_mn, accum=True, out=c), base + res.float(), k)
+    f = torch.ones(m, n, device=dev)
+    gemm(a, b, a_mn=a_mn, b_mn=b_mn, accum=True, out=f)
+    _close(f, base + 1, k)
+    _lib.assert_status_ok("gemm slices")

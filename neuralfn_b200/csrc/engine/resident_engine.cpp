@@ -326,8 +326,13 @@ int forward_layers(block_engine& e, int rows, bool decode, int slot, const int* 
         return -1;
       }
       K(nfn_norm_forward(e.x, e.W(yname(l, "ffn_norm")), nullptr, e.xn, nullptr, nullptr, rows, C, c.norm_eps, 1, c.centered_norms, e.stream));
-      if (gemm(e, e.xn, C, e.W(yname(l, "w_gate_up")), e.ff, 2 * F, rows, 2 * F, C, 0, nullptr, nullptr, 0)) return -1;
-      K(nfn_swiglu_forward(e.ff, 2 * F, e.ffa, F, rows, F, e.stream));
+      const void* wgu = e.W(yname(l, "w_gate_up"));
+      const int fused = rows > 128 && !e.qtype_of.count(wgu) ? nfn_gemm_swiglu(e.xn, C, wgu, C, e.ffa, F, rows, F, C, e.stream) : 0;
+      if (fused < 0) return efail("engine: nfn_gemm_swiglu failed with " + std::to_string(fused));
+      if (!fused) {
+        if (gemm(e, e.xn, C, wgu, e.ff, 2 * F, rows, 2 * F, C, 0, nullptr, nullptr, 0)) return -1;
+        K(nfn_swiglu_forward(e.ff, 2 * F, e.ffa, F, rows, F, e.stream));
+      }
       if (c.sandwich_norms) {
         if (gemm(e, e.ffa, F, e.W(yname(l, "w_down")), e.branch, C, rows, C, F, 0, nullptr, nullptr, 0)) return -1;
         K(nfn_rmsnorm_residual(e.branch, e.W(yname(l, "post_ffn_norm")), e.x, e.x, rows, C, post_eps, c.centered_norms, e.stream));

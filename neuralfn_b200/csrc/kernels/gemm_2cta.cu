@@ -83,7 +83,7 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
                : "memory");
 }
 
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, bool SWIGLU = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P2_THREADS, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                       const __grid_constant__ CUtensorMap tma_c, const __grid_constant__ CUtensorMap tma_aux, const GemmParams p) {
@@ -154,7 +154,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
         tile_mn(p, tile % tiles_mn, tm, tn);
         kb_range(tile / tiles_mn, kb_lo, kb_hi);
         const int m0 = tm * (2 * BM) + (int)rank * BM;
-        const int nb0 = tn * BN + (int)rank * (BN / 2);
+        const int nb0 = SWIGLU ? tn * (BN / 2) + (int)rank * p.n : tn * BN + (int)rank * (BN / 2);  // SWIGLU: gate rows, up rows
         for (int kb = kb_lo; kb < kb_hi; ++kb) {
           if (!mbar_wait_bounded(smem_u32(&empty_bar[stage]), phase ^ 1, cta_abort, p.status, NFN_ERR_WAIT_EMPTY)) {
             ok = false;
@@ -216,6 +216,52 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   } else {
     const uint32_t tempty_leader0 = mapa_shared(smem_u32(&tempty_bar[0]), 0);
     const uint32_t tempty_leader1 = mapa_shared(smem_u32(&tempty_bar[1]), 0);
+    if constexpr (SWIGLU) {
+      // columns 0 - 127 of the accumulator are gates, 128 - 255 the same columns' ups: C = silu(gate) * up from fp32
+      const int q = warp & 3, eh = (warp - 2) >> 2;
+      const bool wide = (p.ldc & 15) == 0 && (reinterpret_cast<uintptr_t>(p.c) & 31) == 0;
+      uint32_t acc = 0, acc_phase = 0;
+      for (int tile = pair; tile < num_tiles; tile += n_pairs) {
+        int tm, tn;
+        tile_mn(p, tile, tm, tn);
+        bool ok = mbar_wait_bounded(smem_u32(&tfull_bar[acc]), acc_phase, cta_abort, p.status, NFN_ERR_WAIT_TMEM_FULL);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        const int row = tm * (2 * BM) + (int)rank * BM + q * 32 + lane;
+        const uint32_t taddr = tmem_base + acc * BN + (static_cast<uint32_t>(q * 32) << 16);
+#pragma unroll 1
+        for (int c = eh; c < BN / 64; c += 2) {
+          const int nc = tn * (BN / 2) + c * 32;
+          if (nc >= p.n) break;
+          uint32_t g[32], u[32];
+          tmem_ld_32x32(taddr + c * 32, g);
+          tmem_ld_32x32(taddr + BN / 2 + c * 32, u);
+          tmem_ld_wait();
+          if (row >= p.m) continue;
+          __nv_bfloat16* cp = static_cast<__nv_bfloat16*>(p.c) + (size_t)row * p.ldc + nc;
+          uint4 o[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            float v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = silu_f(__uint_as_float(g[e * 8 + j])) * __uint_as_float(u[e * 8 + j]);
+            o[e] = pack8_bf16(v);
+          }
+          if (nc + 32 <= p.n) {
+            st_row32_bf16(cp, o, wide);
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (nc + e * 8 < p.n) *reinterpret_cast<uint4*>(cp + e * 8) = o[e];
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(acc ? tempty_leader1 : tempty_leader0);
+        if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+      }
+    } else {
 #define EPI_TILE_FIRST pair
 #define EPI_TILE_STEP n_pairs
 #define EPI_TILE_M0(tm) ((tm) * (2 * BM) + (int)rank * BM)
@@ -225,6 +271,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
 #undef EPI_TILE_STEP
 #undef EPI_TILE_M0
 #undef EPI_RELEASE_ACC
+    }
   }
 
   // ---------------------------------------------------------------- teardown --
@@ -244,14 +291,16 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
 
 namespace nfn {
 
+constexpr size_t P2_SMEM = 1024 + (size_t)P2_STAGES * (P2_BM * P2_BK * 2 + (P2_BN / 2) * P2_BK * 2) + 2 * P2_EPI_TILE + 256;
+
 // CTA pairs that can be resident at the same time (GPCs with an odd number of free SMs leave one SM without a partner)
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, bool SWIGLU = false>
 static int prepare_pair_kernel(size_t smem) {
   static int max_pairs[64] = {};  // per device
   int dev = 0;
   cudaGetDevice(&dev);
   if (!max_pairs[dev & 63]) {
-    auto kern = gemm_bf16_pair_kernel<A_MN, B_MN>;
+    auto kern = gemm_bf16_pair_kernel<A_MN, B_MN, SWIGLU>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return launch_check("gemm_pair attr", 0);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sm_count() & ~1, 1, 1);
@@ -276,7 +325,7 @@ static int prepare_pair_kernel(size_t smem) {
 
 template <bool A_MN, bool B_MN>
 static int launch_pair(const nfn_gemm_args& a, int split_k, cudaStream_t stream, const int* group_rows, int groups, long long group_stride) {
-  constexpr size_t SMEM = 1024 + (size_t)P2_STAGES * (P2_BM * P2_BK * 2 + (P2_BN / 2) * P2_BK * 2) + 2 * P2_EPI_TILE + 256;
+  constexpr size_t SMEM = P2_SMEM;
   const int max_pairs = prepare_pair_kernel<A_MN, B_MN>(SMEM);
   if (max_pairs <= 0) return max_pairs;
   CUtensorMap ta, tb, tc, tx;
@@ -327,6 +376,30 @@ static int launch_pair(const nfn_gemm_args& a, int split_k, cudaStream_t stream,
   const int tiles = p.tiles_m * p.tiles_n * p.split_k;
   launch_overlapped(gemm_bf16_pair_kernel<A_MN, B_MN>, 2 * std::min(max_pairs, tiles), P2_THREADS, SMEM, stream, ta, tb, tc, tx, p);
   const int rc = launch_check("gemm_pair", 1);
+  return rc < 0 ? rc : 1;
+}
+
+// C[M, ff] = silu(A Wg^T) * (A Wu^T) with B = [Wg; Wu] stacked, 2 ff rows: one CTA of the pair stages 128 gate rows, the other the up rows of the
+// same columns, so gates and ups never go to memory. 8191 x 14336 x 4096: @W1@.
+int launch_gemm_pair_swiglu(const nfn_gemm_args& a, int ff, cudaStream_t stream) {
+  const int max_pairs = prepare_pair_kernel<false, false, true>(P2_SMEM);
+  if (max_pairs <= 0) return max_pairs;
+  CUtensorMap ta, tb;
+  if (!make_tmap_2d(&ta, a.a, 2, (uint64_t)a.k, (uint64_t)a.m, (uint64_t)a.lda, P2_BK, P2_BM, 128)) return -3;
+  if (!make_tmap_2d(&tb, a.b, 2, (uint64_t)a.k, 2ull * ff, (uint64_t)a.ldb, P2_BK, P2_BN / 2, 128)) return -3;
+  GemmParams p{};
+  p.c = a.c;
+  p.m = a.m; p.n = ff; p.k = a.k;
+  p.ldc = a.ldc;
+  p.alpha = 1.f;
+  p.tiles_m = ceil_div(a.m, 2 * P2_BM);
+  p.tiles_n = ceil_div(ff, P2_BN / 2);
+  p.split_k = 1;
+  p.kb_per_split = ceil_div(a.k, P2_BK);
+  p.status = status_ptr();
+  p.raster_gw = pick_raster_gw(a.m, a.k, p.tiles_n);
+  launch_overlapped(gemm_bf16_pair_kernel<false, false, true>, 2 * std::min(max_pairs, p.tiles_m * p.tiles_n), P2_THREADS, P2_SMEM, stream, ta, tb, ta, ta, p);
+  const int rc = launch_check("gemm_pair_swiglu", 1);
   return rc < 0 ? rc : 1;
 }
 

@@ -161,6 +161,7 @@ static int launch_gemm(const nfn_gemm_args& a, int split_k, cudaStream_t stream,
 
 // gemm_2cta.cu
 bool gemm_pair_ok(const nfn_gemm_args& a);
+int launch_gemm_pair_swiglu(const nfn_gemm_args& a, int ff, cudaStream_t stream);
 int launch_gemm_pair(const nfn_gemm_args& a, int split_k, cudaStream_t stream, const int* group_rows, int groups, long long group_stride);
 
 // gemm_slices.cu
@@ -277,6 +278,21 @@ extern "C" int nfn_gemm_grouped_k(const nfn_gemm_args* args, const int* group_ro
   const int tiles256 = ceil_div(a.m, BM) * ceil_div(a.n, 256) * groups;
   if (tiles256 >= sm_count() && (a.n % 256 == 0 || a.n >= 1024)) return launch_gemm<256, 4, true, true>(a, 1, stream, group_rows, groups, group_stride);
   return launch_gemm<128, 6, true, true>(a, 1, stream, group_rows, groups, group_stride);
+}
+
+// c [m, ff] = silu(a wg^T) * (a wu^T) for stacked weights b = [wg; wu] (2 ff rows of k), in one launch where the plain product would run on
+// CTA pairs: 1. 0: not such a product, nothing was launched and the caller runs the product and nfn_swiglu_forward. < 0: error.
+extern "C" int nfn_gemm_swiglu(const void* x, int ldx, const void* b, int ldb, void* c, int ldc, int m, int ff, int k, nfn_stream_t stream) {
+  using namespace nfn;
+  if (m <= 128 || ff <= 0 || k <= 0 || !pair_enabled() || ((ff | ldx | ldb | ldc) & 7) || ff < 128) return 0;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) return 0;
+  nfn_gemm_args a{};
+  a.a = x; a.b = b; a.c = c;
+  a.m = m; a.n = 2 * ff; a.k = k;
+  a.lda = ldx; a.ldb = ldb; a.ldc = ldc;
+  a.alpha = 1.f; a.split_k = 1;
+  if (plan_gemm(a, sm_count(), true, false, 0).tile != TILE_PAIR) return 0;
+  return launch_gemm_pair_swiglu(a, ff, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int nfn_gemm_bf16(const nfn_gemm_args* args, nfn_stream_t stream_) {

@@ -67,6 +67,7 @@ typedef struct {
   void* workspace; long long workspace_bytes; int split_k;
 } nfn_gemm_args;
 
+int nfn_gemm_swiglu(const void* x, int ldx, const void* b, int ldb, void* c, int ldc, int m, int ff, int k, nfn_stream_t stream);
 int nfn_gemm_bf16(const nfn_gemm_args* args, nfn_stream_t stream);
 // Grouped contraction for expert weight gradients: C[g] = A[K rows of group g, M]^T . B[same rows, N] for every group in one
 // launch. Both operands MN-major; group_rows = groups + 1 device ints (multiples of 64; padding rows zero); C slices

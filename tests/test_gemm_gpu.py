@@ -357,3 +357,22 @@ def test_gemm_slices_in_a_cluster(kernel_lib, a_mn, b_mn, m, n, k):
     gemm(a, b, a_mn=a_mn, b_mn=b_mn, accum=True, out=f)
     _close(f, base + 1, k)
     _lib.assert_status_ok("gemm slices")
+
+
+@pytest.mark.parametrize("m,ff,k", [(8191, 1048, 512), (4100, 3000, 1032), (2056, 11272, 520)])
+def test_gemm_swiglu(kernel_lib, m, ff, k):
+    """Gate and up of a column in one pair tile: a last column tile that runs from the gates into the ups, row and k remainders. One rounding to bf16 of
+    fp32 values."""
+    import ctypes
+    from neuralfn_b200.ops import _lib
+    torch.manual_seed(m)
+    x, w = torch.randn(m, k, device="cuda").bfloat16(), (torch.randn(2 * ff, k, device="cuda") * k ** -0.5).bfloat16()
+    out = torch.full((m + 1, ff + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    P, I = ctypes.c_void_p, ctypes.c_int
+    rc = _lib.load().nfn_gemm_swiglu(P(x.data_ptr()), I(k), P(w.data_ptr()), I(k), P(out.data_ptr()), I(ff + 8), I(m), I(ff), I(k), P(_lib.stream_ptr()))
+    assert rc == 1
+    g, u = (x.double() @ w.double().T).split(ff, -1)
+    ref = torch.nn.functional.silu(g) * u
+    _lib.assert_status_ok("gemm_swiglu")
+    assert bool(((out[:m, :ff].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4).all())
+    assert bool((out[m:] == 7).all()) and bool((out[:, ff:] == 7).all())

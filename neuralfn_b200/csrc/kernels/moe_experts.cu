@@ -43,7 +43,7 @@ moe_index_kernel(const long long* __restrict__ experts, int n, int E, int* __res
   if (i < n) {
     const long long v = experts[i];
     if (v >= 0 && v < E) e = (int)v;
-    else *bad = 1;                                    // host-mapped: the call is refused
+    else if (bad) *bad = 1;                           // host-mapped: the call is refused
   }
   const unsigned same = __match_any_sync(0xffffffffu, e);
   const int before = __popc(same & ((1u << lane) - 1u));
@@ -539,11 +539,11 @@ extern "C" int nfn_moe_experts_forward(const nfn_moe_experts_args* args, nfn_str
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   cudaStreamIsCapturing(stream, &capture);
   const bool eager = capture == cudaStreamCaptureStatusNone;
-  *bad.host = 0;
+  if (eager) *bad.host = 0;
 
   const int n = a.tokens * a.top, blocks = ceil_div(n, MX_IDX);
   const long long pad = (long long)a.experts * (MX_TILE - 1);
-  moe_index_kernel<<<blocks, MX_IDX, 0, stream>>>(a.indices, n, a.experts, ints(at.rank), ints(at.first), bad.dev);
+  moe_index_kernel<<<blocks, MX_IDX, 0, stream>>>(a.indices, n, a.experts, ints(at.rank), ints(at.first), eager ? bad.dev : nullptr);  // a replay must not touch this thread's word
   if (eager) cudaEventRecord(bad.done, stream);
   moe_segments_kernel<<<1, 1024, 0, stream>>>(ints(at.first), blocks, a.experts, a.capacity_rows / MX_TILE, ints(at.offsets), ints(at.rows),
                                               ints(at.tile_expert), ints(at.plan));

@@ -235,6 +235,7 @@ int forward_layers(block_engine& e, int rows, bool decode, int slot, const int* 
     CU(cudaMemcpyAsync(e.tq_idx, idx.data(), idx.size() * 4, cudaMemcpyHostToDevice, e.stream));
     CU(cudaStreamSynchronize(e.stream));  // `idx` leaves scope
   }
+  bool normed = false;  // e.xn already holds this layer's attention norm
   for (int l = 0; l < c.n_layer; ++l) {
     const bool local = layer_is_local(c, l);
     const int cap = e.cap[l];
@@ -246,10 +247,12 @@ int forward_layers(block_engine& e, int rows, bool decode, int slot, const int* 
       K(nfn_norm_forward(e.x, e.W(gname(l, "ln_1.weight")), e.W(gname(l, "ln_1.bias")), e.xn, nullptr, nullptr, rows, C, c.norm_eps, 0, 0, e.stream));
       if (gemm(e, e.xn, C, e.W(gname(l, "attn.c_attn.weight")), e.qkv, e.qkv_ld, rows, e.qkv_ld, C, 0, e.W(gname(l, "attn.c_attn.bias")), nullptr, 0)) return -1;
     } else {
-      K(nfn_norm_forward(e.x, e.W(yname(l, "attn_norm")), nullptr, e.xn, nullptr, nullptr, rows, C, c.norm_eps, 1, c.centered_norms, e.stream));
+      if (!normed) K(nfn_norm_forward(e.x, e.W(yname(l, "attn_norm")), nullptr, e.xn, nullptr, nullptr, rows, C, c.norm_eps, 1, c.centered_norms, e.stream));
       if (gemm(e, e.xn, C, e.W(yname(l, "wqkv")), e.qkv, e.qkv_ld, rows, e.qkv_ld, C, 0, nullptr, nullptr, 0)) return -1;
       if (c.qk_norm == 2) { qw = e.W(yname(l, "q_norm")); kw = e.W(yname(l, "k_norm")); }
     }
+    // the prompt's attention applies the output gate in its epilogue where the packed rows keep it 16-byte aligned
+    const bool gate_in_attention = c.family == 1 && c.gated_attention && !decode && block_rows == 0 && (e.qkv_ld & 7) == 0;
     const bool rope = c.family == 1 && (!c.rope_local_only || local);
     const float q_scale = (c.family == 1 && c.q_scale > 0.f) ? c.q_scale : 1.f;
     if (decode && e.tq) {
@@ -297,8 +300,13 @@ int forward_layers(block_engine& e, int rows, bool decode, int slot, const int* 
                               Hkv, HD, cap, local ? cap : 0, 1, scale, e.blk_ws, e.blk_ws_bytes, 0, e.stream));
       } else {
         const char* q = static_cast<const char*>(e.qkv);
-        K(nfn_attention_forward(q, q + (size_t)Hq * HD * 2, q + (size_t)(Hq + Hkv) * HD * 2, e.att, nullptr, 1, rows, Hq, Hkv, HD, e.qkv_ld,
-                                e.qkv_ld, e.qkv_ld, ATT, 1, local ? c.window : 0, scale, e.stream));
+        nfn_attention_args at{};
+        at.q = q; at.k = q + (size_t)Hq * HD * 2; at.v = q + (size_t)(Hq + Hkv) * HD * 2; at.o = e.att;
+        at.B = 1; at.T = rows; at.Hq = Hq; at.Hkv = Hkv; at.D = HD;
+        at.ld_q = at.ld_k = at.ld_v = e.qkv_ld; at.ld_o = ATT;
+        at.causal = 1; at.window = local ? c.window : 0; at.scale = scale;
+        if (gate_in_attention) { at.gate = q + (size_t)(Hq + 2 * Hkv) * HD * 2; at.ld_gate = e.qkv_ld; }
+        K(nfn_attention_forward_ex(&at, e.stream));
         if (e.tq) {
           const int* d_slot = e.tq_idx + (local ? rows : 2 * rows);
           K(nfn_turboquant_encode(&e.tq_tables, q + (size_t)Hq * HD * 2, e.qkv_ld, e.tq_idx, d_slot, rows, Hkv, cap, 1, kc, e.stream));
@@ -315,17 +323,18 @@ int forward_layers(block_engine& e, int rows, bool decode, int slot, const int* 
       if (gemm(e, e.ff, F, e.W(gname(l, "mlp.c_proj.weight")), e.x, C, rows, C, F, 0, e.W(gname(l, "mlp.c_proj.bias")), e.x, C)) return -1;
     } else {
       const float post_eps = c.post_norm_eps > 0.f ? c.post_norm_eps : c.norm_eps;
-      if (c.gated_attention) {
+      if (c.gated_attention && !gate_in_attention) {
         const char* gate = static_cast<const char*>(e.qkv) + (size_t)(Hq + 2 * Hkv) * HD * 2;
         K(nfn_sigmoid_gate_inplace(e.att, ATT, gate, e.qkv_ld, rows, ATT, e.stream));
       }
       if (c.sandwich_norms) {
         if (gemm(e, e.att, ATT, e.W(yname(l, "wo")), e.branch, C, rows, C, ATT, 0, nullptr, nullptr, 0)) return -1;
-        K(nfn_rmsnorm_residual(e.branch, e.W(yname(l, "post_attn_norm")), e.x, e.x, rows, C, post_eps, c.centered_norms, e.stream));
+        K(nfn_rmsnorm_residual_norm(e.branch, e.W(yname(l, "post_attn_norm")), e.x, e.x, e.W(yname(l, "ffn_norm")), e.xn, rows, C, post_eps, c.norm_eps,
+                                    c.centered_norms, e.stream));
       } else if (gemm(e, e.att, ATT, e.W(yname(l, "wo")), e.x, C, rows, C, ATT, 0, nullptr, e.x, C)) {
         return -1;
       }
-      K(nfn_norm_forward(e.x, e.W(yname(l, "ffn_norm")), nullptr, e.xn, nullptr, nullptr, rows, C, c.norm_eps, 1, c.centered_norms, e.stream));
+      if (!c.sandwich_norms) K(nfn_norm_forward(e.x, e.W(yname(l, "ffn_norm")), nullptr, e.xn, nullptr, nullptr, rows, C, c.norm_eps, 1, c.centered_norms, e.stream));
       const void* wgu = e.W(yname(l, "w_gate_up"));
       const int fused = rows > 128 && !e.qtype_of.count(wgu) ? nfn_gemm_swiglu(e.xn, C, wgu, C, e.ffa, F, rows, F, C, e.stream) : 0;
       if (fused < 0) return efail("engine: nfn_gemm_swiglu failed with " + std::to_string(fused));
@@ -335,7 +344,12 @@ int forward_layers(block_engine& e, int rows, bool decode, int slot, const int* 
       }
       if (c.sandwich_norms) {
         if (gemm(e, e.ffa, F, e.W(yname(l, "w_down")), e.branch, C, rows, C, F, 0, nullptr, nullptr, 0)) return -1;
-        K(nfn_rmsnorm_residual(e.branch, e.W(yname(l, "post_ffn_norm")), e.x, e.x, rows, C, post_eps, c.centered_norms, e.stream));
+        normed = l + 1 < c.n_layer;
+        if (normed)
+          K(nfn_rmsnorm_residual_norm(e.branch, e.W(yname(l, "post_ffn_norm")), e.x, e.x, e.W(yname(l + 1, "attn_norm")), e.xn, rows, C, post_eps, c.norm_eps,
+                                      c.centered_norms, e.stream));
+        else
+          K(nfn_rmsnorm_residual(e.branch, e.W(yname(l, "post_ffn_norm")), e.x, e.x, rows, C, post_eps, c.centered_norms, e.stream));
       } else if (gemm(e, e.ffa, F, e.W(yname(l, "w_down")), e.x, C, rows, C, F, 0, nullptr, e.x, C)) {
         return -1;
       }

@@ -67,6 +67,9 @@ typedef struct {
   void* workspace; long long workspace_bytes; int split_k;
 } nfn_gemm_args;
 
+// x_out = resid + RMS(x) * weight, y = RMS(x_out) * weight_next (1 + w each when centered)
+int nfn_rmsnorm_residual_norm(const void* x, const void* weight, const void* resid, void* x_out, const void* weight_next, void* y, long long rows, int C,
+                              float eps, float eps_next, int centered, nfn_stream_t stream);
 int nfn_gemm_swiglu(const void* x, int ldx, const void* b, int ldb, void* c, int ldc, int m, int ff, int k, nfn_stream_t stream);
 int nfn_gemm_bf16(const nfn_gemm_args* args, nfn_stream_t stream);
 // Grouped contraction for expert weight gradients: C[g] = A[K rows of group g, M]^T . B[same rows, N] for every group in one

@@ -392,3 +392,20 @@ def test_nf4_lora_linear_fused_forward_and_backward(kernel_lib, M, N, K, r):
     db_ref = s * dyf.T @ (xf @ Af.T)
     for got, want in ((dx.float(), dx_ref), (da, da_ref), (db, db_ref)):
         torch.testing.assert_close(got, want, atol=0.03 * float(want.abs().max()), rtol=3e-2)
+
+
+@pytest.mark.parametrize("rows,C,centered", [(1, 8, False), (3, 2048, True), (5, 2056, True), (2, 4104, False), (3, 8192, True)])
+def test_rmsnorm_residual_norm_equals_the_two_passes(kernel_lib, rows, C, centered):
+    """In place over the residual, at the ends of each register count: the values of the two launches up to the order of a row's fp32 sum (one bf16 step)."""
+    import ctypes
+    from neuralfn_b200.ops import _lib, infer, kernels as K
+    torch.manual_seed(C)
+    x, res, w1, w2 = (torch.randn(*s, device="cuda").bfloat16() for s in ((rows, C), (rows, C), (C,), (C,)))
+    want = infer.rmsnorm_residual(x, w1, res, eps=1e-6, centered=centered)
+    y, P = torch.empty_like(x), lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    rc = _lib.load().nfn_rmsnorm_residual_norm(P(x), P(w1), P(res), P(res), P(w2), P(y), ctypes.c_longlong(rows), ctypes.c_int(C), ctypes.c_float(1e-6),
+                                               ctypes.c_float(1e-5), ctypes.c_int(int(centered)), ctypes.c_void_p(_lib.stream_ptr()))
+    assert rc == 0
+    want_y, _, _ = K.norm_forward(res, w2, None, mode=K.NORM_RMS, eps=1e-5, centered=centered)   # of the sum as stored: a step there is not a step here
+    for a, b in ((res, want), (y, want_y)):
+        assert bool(((a.float() - b.float()).abs() <= 2.0 ** -7 * b.float().abs() + 1e-6).all())

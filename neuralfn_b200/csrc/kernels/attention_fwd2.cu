@@ -134,6 +134,8 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_trigger();
+  grid_wait();
   const int row0 = b * T;  // first token row of this batch in the [B*T, width] views
 
   if (warp == AV2_TMA_WARP) {
@@ -233,7 +235,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     constexpr bool capped = (FEAT & AF_SOFTCAP) != 0;
     const float cap_in = capped ? p.scale / p.softcap : 0.f;
     const float c_mul = capped ? p.softcap * LOG2E : p.scale * LOG2E;
-    const int my_seq = ((FEAT & AF_SEQ) && q < T) ? __ldg(p.mask.seq_ids + row0 + q) : 0;
+    const int my_seq = ((FEAT & AF_SEQ) && q < T) ? *(p.mask.seq_ids + row0 + q) : 0;
     // visible keys of this row form one interval [v_lo, v_hi)
     int v_lo = 0, v_hi = T;
     if (p.mask.causal) {
@@ -276,7 +278,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
           for (int i = 0; i < BN; ++i) {
             const int k = min(kbase + i, T - 1);
-            if (__ldg(p.mask.seq_ids + row0 + k) != my_seq) s[i] = 0xff800000u;
+            if (*(p.mask.seq_ids + row0 + k) != my_seq) s[i] = 0xff800000u;
           }
         }
       }
@@ -455,7 +457,7 @@ static int launch_attn_fwd2(const nfn_attention_args& a, cudaStream_t st) {
   p.scale = a.scale; p.softcap = a.softcap;
   p.status = status_ptr();
   dim3 grid(ceil_div(a.T, C::BM), a.Hq, a.B);
-  kern<<<grid, AV2_THREADS, SMEM, st>>>(tq, tk, tv, p);
+  launch_overlapped(kern, grid, AV2_THREADS, SMEM, st, tq, tk, tv, p);
   return launch_check("attn_fwd2");
 }
 

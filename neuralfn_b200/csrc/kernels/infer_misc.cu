@@ -60,9 +60,11 @@ swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, int ld, const __nv_bfloa
 }
 
 __global__ void __launch_bounds__(256)
-embedding_pos_kernel(const int* __restrict__ tokens, const int* __restrict__ positions, const __nv_bfloat16* __restrict__ wte,
-                     const __nv_bfloat16* __restrict__ wpe, __nv_bfloat16* __restrict__ out, int n, int C, int vocab, int max_pos,
+embedding_pos_kernel(const int* tokens, const int* positions, const __nv_bfloat16* wte,
+                     const __nv_bfloat16* wpe, __nv_bfloat16* out, int n, int C, int vocab, int max_pos,
                      float scale) {
+  grid_trigger();
+  grid_wait();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int vecs = C / 8;
   if (idx >= (long long)n * vecs) return;
@@ -86,8 +88,10 @@ embedding_pos_kernel(const int* __restrict__ tokens, const int* __restrict__ pos
 
 // rows t in [t_first, n): k/v heads of row t -> cache slot (pos0 + t) % cap
 __global__ void __launch_bounds__(256)
-kv_cache_write_kernel(const __nv_bfloat16* __restrict__ qkv, int ld, __nv_bfloat16* __restrict__ kc, __nv_bfloat16* __restrict__ vc,
+kv_cache_write_kernel(const __nv_bfloat16* qkv, int ld, __nv_bfloat16* kc, __nv_bfloat16* vc,
                       int n, int t_first, int Hq, int Hkv, int hd, int cap, int pos0) {
+  grid_trigger();
+  grid_wait();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int vecs = hd / 8;
   const long long total = (long long)(n - t_first) * Hkv * vecs;
@@ -136,8 +140,7 @@ extern "C" int nfn_embedding_positions(const int* tokens, const int* positions, 
   if (n <= 0) return 0;
   if (!tokens || !wte || !out || (wpe && !positions) || C <= 0 || (C & 7) || vocab <= 0) return fail(-1, "embedding_positions: bad arguments");
   const long long total = (long long)n * (C / 8);
-  embedding_pos_kernel<<<(unsigned)((total + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      tokens, positions, static_cast<const __nv_bfloat16*>(wte), static_cast<const __nv_bfloat16*>(wpe),
+  launch_overlapped(embedding_pos_kernel, (unsigned)((total + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream), tokens, positions, static_cast<const __nv_bfloat16*>(wte), static_cast<const __nv_bfloat16*>(wpe),
       static_cast<__nv_bfloat16*>(out), n, C, vocab, max_pos > 0 ? max_pos : 1, scale);
   return launch_check("embedding_positions", 1);
 }
@@ -149,8 +152,7 @@ extern "C" int nfn_kv_cache_write(const void* qkv, int ld, void* k_cache, void* 
     return fail(-1, "kv_cache_write: bad arguments");
   const int t_first = n > cap ? n - cap : 0;  // earlier rows would be overwritten anyway (and would race)
   const long long total = (long long)(n - t_first) * n_kv_heads * (head_dim / 8);
-  kv_cache_write_kernel<<<(unsigned)((total + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(qkv), ld, static_cast<__nv_bfloat16*>(k_cache), static_cast<__nv_bfloat16*>(v_cache), n,
+  launch_overlapped(kv_cache_write_kernel, (unsigned)((total + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(qkv), ld, static_cast<__nv_bfloat16*>(k_cache), static_cast<__nv_bfloat16*>(v_cache), n,
       t_first, n_q_heads, n_kv_heads, head_dim, cap, pos0);
   return launch_check("kv_cache_write", 1);
 }

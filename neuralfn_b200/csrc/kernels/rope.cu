@@ -19,9 +19,11 @@ namespace nfn {
 
 // one thread: 2 low + 2 high elements of one head
 __global__ void __launch_bounds__(256)
-rope_inplace_kernel(__nv_bfloat16* __restrict__ qkv, int ld, long long n_items, int T, int heads, int hd, int rot_dim,
-                    const float* __restrict__ cosT, const float* __restrict__ sinT, const int* __restrict__ positions,
+rope_inplace_kernel(__nv_bfloat16* qkv, int ld, long long n_items, int T, int heads, int hd, int rot_dim,
+                    const float* cosT, const float* sinT, const int* positions,
                     int max_pos, float sign, float q_scale, int n_q_heads) {
+  grid_trigger();
+  grid_wait();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n_items) return;
   const int half = rot_dim >> 1, per_head = half >> 1;
@@ -48,10 +50,12 @@ rope_inplace_kernel(__nv_bfloat16* __restrict__ qkv, int ld, long long n_items, 
 
 // one warp per (token, head); hd in {64, 128}; lane l owns low pair 2l and high pair half+2l
 __global__ void __launch_bounds__(256)
-qk_norm_rope_kernel(__nv_bfloat16* __restrict__ qkv, int ld, long long n_rows, int T, int heads, int hd,
-                    const __nv_bfloat16* __restrict__ q_weight, const __nv_bfloat16* __restrict__ k_weight,
-                    const float* __restrict__ cosT, const float* __restrict__ sinT, const int* __restrict__ positions,
-                    int max_pos, float sign, float eps, float q_scale, int n_q_heads, float* __restrict__ rstd_out) {
+qk_norm_rope_kernel(__nv_bfloat16* qkv, int ld, long long n_rows, int T, int heads, int hd,
+                    const __nv_bfloat16* q_weight, const __nv_bfloat16* k_weight,
+                    const float* cosT, const float* sinT, const int* positions,
+                    int max_pos, float sign, float eps, float q_scale, int n_q_heads, float* rstd_out) {
+  grid_trigger();
+  grid_wait();
   const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= n_rows) return;
   const int lane = threadIdx.x & 31, half = hd >> 1, per_head = half >> 1;
@@ -111,8 +115,7 @@ extern "C" int nfn_rope_inplace(void* qkv, int ld, long long tokens, int T, int 
   const long long items = tokens * heads * (rot_dim / 4);
   const long long blocks = (items + 255) / 256;
   if (blocks > 0x7fffffffLL) return fail(-1, "rope: too many elements for one launch");
-  rope_inplace_kernel<<<(unsigned)blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<__nv_bfloat16*>(qkv), ld, items, T, heads, head_dim, rot_dim, cos_table, sin_table, positions, max_pos, sign,
+  launch_overlapped(rope_inplace_kernel, (unsigned)blocks, 256, 0, static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(qkv), ld, items, T, heads, head_dim, rot_dim, cos_table, sin_table, positions, max_pos, sign,
       q_scale, n_q_heads);
   return launch_check("rope_inplace", 1);
 }
@@ -126,8 +129,7 @@ extern "C" int nfn_qk_norm_rope_forward(void* qkv, int ld, long long tokens, int
   const long long rows = tokens * (n_q_heads + n_kv_heads);
   const long long blocks = (rows + 7) / 8;
   if (blocks > 0x7fffffffLL) return fail(-1, "qk_norm_rope: too many rows for one launch");
-  qk_norm_rope_kernel<<<(unsigned)blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<__nv_bfloat16*>(qkv), ld, rows, T, n_q_heads + n_kv_heads, head_dim,
+  launch_overlapped(qk_norm_rope_kernel, (unsigned)blocks, 256, 0, static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(qkv), ld, rows, T, n_q_heads + n_kv_heads, head_dim,
       static_cast<const __nv_bfloat16*>(q_weight), static_cast<const __nv_bfloat16*>(k_weight), cos_table, sin_table, positions,
       max_pos, sign, eps, q_scale, n_q_heads, rstd_out);
   return launch_check("qk_norm_rope_forward", 1);

@@ -336,7 +336,7 @@ int forward_layers(block_engine& e, int rows, bool decode, int slot, const int* 
       }
       if (!c.sandwich_norms) K(nfn_norm_forward(e.x, e.W(yname(l, "ffn_norm")), nullptr, e.xn, nullptr, nullptr, rows, C, c.norm_eps, 1, c.centered_norms, e.stream));
       const void* wgu = e.W(yname(l, "w_gate_up"));
-      const int fused = rows > 128 && !e.qtype_of.count(wgu) ? nfn_gemm_swiglu(e.xn, C, wgu, C, e.ffa, F, rows, F, C, e.stream) : 0;
+      const int fused = e.qtype_of.count(wgu) ? 0 : nfn_gemm_swiglu(e.xn, C, wgu, C, e.ffa, F, rows, F, C, 1, e.stream);
       if (fused < 0) return efail("engine: nfn_gemm_swiglu failed with " + std::to_string(fused));
       if (!fused) {
         if (gemm(e, e.xn, C, wgu, e.ff, 2 * F, rows, 2 * F, C, 0, nullptr, nullptr, 0)) return -1;

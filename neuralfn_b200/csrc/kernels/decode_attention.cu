@@ -381,7 +381,7 @@ decode_attention_kernel(const DecodeParams p) {
 // are prepared, the next K rows as soon as the scores have consumed the last, and the merge of the splits works from
 // weights that are computed once, its loads independent of each other.
 // Per launch, 1 sequence of 1023, 16 query heads of 128 on 4: 16.6 -> 9.1 us; 4 of up to 2047: 22.3 -> 11.5 us; 32 of 128 - 3071, 32 heads
-// on 8: 81.6 -> 52.4 us (3.6 TB/s).
+// on 8: 81.6 -> 43.4 us (4.3 TB/s).
 constexpr int MMA_WARPS = 4;
 constexpr int MMA_STEP = 16;  // positions per warp step
 
@@ -844,11 +844,12 @@ extern "C" int nfn_decode_attention(const void* qkv, int ld, void* k_cache, void
     const long long want = ((use_mma ? 3LL : 2LL) * sm_count()) / units;
     splits = (int)std::max<long long>(1, std::min<long long>(want, (cap + 127) / 128));
     if (use_mma) {
-      // Cut by the sequence: 64 positions (one step per warp) while the launch is a matter of latency, up to 256 (four
-      // steps) when there are many units, so that preparing the queries does not outweigh the stream. As many
-      // splits as the workspace holds, at least the number above.
+      // Cut by the sequence: 64 positions (one step per warp) while the launch is a matter of latency, up to 512 (eight steps) when
+      // there are many units, so that preparing the queries does not outweigh the stream (32 x 8 units of up to 3071: 64 98 us,
+      // 128 66, 256 51, 512 43, 1024 45; 4 units of 1023: 64 9.0, 256 10.9, 512 12.4). As many splits as the workspace holds, at
+      // least the number above.
       chunk = 64;
-      while (chunk < 256 && units * ((cap + chunk - 1) / chunk) > 6LL * sm_count()) chunk *= 2;
+      while (chunk < 512 && units * ((cap + chunk - 1) / chunk) > 6LL * sm_count()) chunk *= 2;
       const long long fit = std::min<long long>(64, (workspace_bytes - ticket_bytes) / split_bytes);
       splits = (int)std::max<long long>(splits, std::min<long long>(fit, (cap + chunk - 1) / chunk));
     }

@@ -171,6 +171,7 @@ int gemm_slices_resident(int slices);
 // CTA-pair (cta_group::2) kernel: -1 = read NFN_GEMM_PAIR once.
 static int g_pair_mode = -1;
 int try_launch_gemv(const nfn_gemm_args& a, cudaStream_t stream);  // gemv_bf16.cu
+int launch_gemv_swiglu(const nfn_gemm_args& a, int ff, cudaStream_t stream);  // gemv_bf16.cu
 int try_launch_skinny(const nfn_gemm_args& a, cudaStream_t stream);  // gemm_skinny.cu
 static int g_gemv_mode = 1;
 static int gemv_mode() { return g_gemv_mode; }
@@ -280,17 +281,21 @@ extern "C" int nfn_gemm_grouped_k(const nfn_gemm_args* args, const int* group_ro
   return launch_gemm<128, 6, true, true>(a, 1, stream, group_rows, groups, group_stride);
 }
 
-// c [m, ff] = silu(a wg^T) * (a wu^T) for stacked weights b = [wg; wu] (2 ff rows of k), in one launch where the plain product would run on
-// CTA pairs: 1. 0: not such a product, nothing was launched and the caller runs the product and nfn_swiglu_forward. < 0: error.
-extern "C" int nfn_gemm_swiglu(const void* x, int ldx, const void* b, int ldb, void* c, int ldc, int m, int ff, int k, nfn_stream_t stream) {
+// c [m, ff] = silu(x wg^T) * (x wu^T) for stacked weights b = [wg; wu] (2 ff rows of k), in one launch for one or two rows and where the plain
+// product would run on CTA pairs: 1. 0: not such a product, nothing was launched and the caller runs the product and nfn_swiglu_forward.
+// < 0: error. resident: as NFN_GEMM_STATIC_B.
+extern "C" int nfn_gemm_swiglu(const void* x, int ldx, const void* b, int ldb, void* c, int ldc, int m, int ff, int k, int resident, nfn_stream_t stream) {
   using namespace nfn;
-  if (m <= 128 || ff <= 0 || k <= 0 || !pair_enabled() || ((ff | ldx | ldb | ldc) & 7) || ff < 128) return 0;
+  if (m <= 0 || ff < 128 || k < 64 || ((ff | k | ldx | ldb | ldc) & 7)) return 0;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) return 0;
   nfn_gemm_args a{};
   a.a = x; a.b = b; a.c = c;
   a.m = m; a.n = 2 * ff; a.k = k;
   a.lda = ldx; a.ldb = ldb; a.ldc = ldc;
   a.alpha = 1.f; a.split_k = 1;
+  a.flags = resident ? NFN_GEMM_STATIC_B : 0;
+  if (m <= 2 && gemv_mode() != 0) return launch_gemv_swiglu(a, ff, static_cast<cudaStream_t>(stream));
+  if (m <= 128 || !pair_enabled()) return 0;
   if (plan_gemm(a, sm_count(), true, false, 0).tile != TILE_PAIR) return 0;
   return launch_gemm_pair_swiglu(a, ff, static_cast<cudaStream_t>(stream));
 }

@@ -22,7 +22,7 @@ struct GemvParams {
   __nv_bfloat16* copy;    // out_f32: optional bf16 copy of the result
   const __nv_bfloat16* bias;
   const __nv_bfloat16* resid;
-  int n, k, lda, ldb, ldc, ld_resid, ld_copy;
+  int n, k, lda, ldb, ldc, ld_resid, ld_copy;   // GATED: n columns of gates, their ups n weight rows further
   int act, accum, out_f32;
   int static_b;           // weights may be fetched before the launch ahead of this one is complete
   float alpha, act_param;
@@ -58,19 +58,20 @@ __device__ __forceinline__ float gemv_dot8(const uint4& w, const float (&x)[8]) 
 // CTAs so that every one gets the same number of pairs.
 // Weights of a resident model do not wait for the launch before: the first eight loads of every warp are in flight while that
 // launch still runs, and only the token vectors are read after it.
-template <int M, int KS>
+// GATED: the pair is a gate row and the up row of the same column, and the result is silu(gate) * up.
+template <int M, int KS, bool GATED>
 __global__ void __launch_bounds__(GEMV_THREADS, 3)
 gemv_bf16_kernel(const GemvParams p) {
   constexpr int WARPS = GEMV_THREADS / 32, SLOTS = WARPS / KS;        // row pairs a CTA works on at a time
   __shared__ float part[2][WARPS][2 * M];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = warp % KS;
-  const int pairs = (p.n + 1) >> 1;
+  const int pairs = GATED ? p.n : (p.n + 1) >> 1;
   // this warp's part of K, in chunks of 256
   const int chunks = (p.k + 255) >> 8, k_lo = chunks * sub / KS * 256, k_hi = min(p.k, chunks * (sub + 1) / KS * 256);
   uint4 va[GEMV_UNROLL], vb[GEMV_UNROLL];
   auto load = [&](int pr, int k0) {
-    const __nv_bfloat16* wa = p.b + (size_t)(2 * pr) * p.ldb;
-    const __nv_bfloat16* wb = 2 * pr + 1 < p.n ? wa + p.ldb : wa;     // an odd last row is read twice, its second result dropped
+    const __nv_bfloat16* wa = p.b + (size_t)(GATED ? pr : 2 * pr) * p.ldb;
+    const __nv_bfloat16* wb = GATED ? wa + (size_t)p.n * p.ldb : 2 * pr + 1 < p.n ? wa + p.ldb : wa;     // an odd last row is read twice, its second result dropped
 #pragma unroll
     for (int u = 0; u < GEMV_UNROLL; ++u) {
       const int k = k0 + u * 256;
@@ -113,7 +114,7 @@ gemv_bf16_kernel(const GemvParams p) {
 #pragma unroll
         for (int s = 16; s > 0; s >>= 1) acc[r][m] += __shfl_xor_sync(0xffffffffu, acc[r][m], s);
     // lane (r * M + m) finishes output (row m, column n0 + r)
-    const int r = lane / M, m = lane % M, n = 2 * pr + r;
+    const int r = lane / M, m = lane % M, n = GATED ? pr : 2 * pr + r;
     float v = 0.f;
 #pragma unroll
     for (int rr = 0; rr < 2; ++rr)
@@ -128,7 +129,10 @@ gemv_bf16_kernel(const GemvParams p) {
 #pragma unroll
         for (int q = 0; q < KS; ++q) v += part[it & 1][warp - sub + q][lane];
     }
-    if (lane < 2 * M && sub == 0 && n < p.n) {
+    if constexpr (GATED) {
+      const float up = __shfl_sync(0xffffffffu, v, (lane + M) & 31);
+      if (lane < M && sub == 0 && n < p.n) static_cast<__nv_bfloat16*>(p.c)[(size_t)m * p.ldc + n] = __float2bfloat16(silu_f(v) * up);
+    } else if (lane < 2 * M && sub == 0 && n < p.n) {
       v *= p.alpha;
       if (p.bias) v += __bfloat162float(p.bias[n]);
       v = gemv_act(v, p.act, p.act_param);
@@ -147,14 +151,14 @@ gemv_bf16_kernel(const GemvParams p) {
   }
 }
 
-template <int KS>
+template <int KS, bool GATED = false>
 static void launch_gemv_bf16(const GemvParams& p, int m, cudaStream_t stream) {
   // as many CTAs as three per SM, trimmed so that every one takes the same number of row pairs
   constexpr int SLOTS = GEMV_THREADS / 32 / KS;
-  const int items = ((p.n + 1) / 2 + SLOTS - 1) / SLOTS, resident = sm_count() * 3, rounds = (items + resident - 1) / resident;
+  const int items = ((GATED ? p.n : (p.n + 1) / 2) + SLOTS - 1) / SLOTS, resident = sm_count() * 3, rounds = (items + resident - 1) / resident;
   const int grid = (items + rounds - 1) / rounds;
-  if (m == 1) launch_overlapped(gemv_bf16_kernel<1, KS>, grid, GEMV_THREADS, 0, stream, p);
-  else launch_overlapped(gemv_bf16_kernel<2, KS>, grid, GEMV_THREADS, 0, stream, p);
+  if (m == 1) launch_overlapped(gemv_bf16_kernel<1, KS, GATED>, grid, GEMV_THREADS, 0, stream, p);
+  else launch_overlapped(gemv_bf16_kernel<2, KS, GATED>, grid, GEMV_THREADS, 0, stream, p);
 }
 
 // Returns 1 when it launched, 0 when the product is not a GEMV case (the caller continues with the
@@ -185,6 +189,23 @@ int try_launch_gemv(const nfn_gemm_args& a, cudaStream_t stream) {
   else if (narrow && a.k >= 512) launch_gemv_bf16<2>(p, a.m, stream);
   else launch_gemv_bf16<1>(p, a.m, stream);
   const int rc = launch_check("gemv_bf16", 1);
+  return rc == 0 ? 1 : rc;
+}
+
+// c [m, ff] = silu(a wg^T) * (a wu^T), b = [wg; wu], m <= 2; the warps per row pair as for a product of 2 ff columns.
+int launch_gemv_swiglu(const nfn_gemm_args& a, int ff, cudaStream_t stream) {
+  GemvParams p{};
+  p.a = static_cast<const __nv_bfloat16*>(a.a);
+  p.b = static_cast<const __nv_bfloat16*>(a.b);
+  p.c = a.c;
+  p.n = ff; p.k = a.k; p.lda = a.lda; p.ldb = a.ldb; p.ldc = a.ldc;
+  p.alpha = 1.f;
+  p.static_b = (a.flags & NFN_GEMM_STATIC_B) ? 1 : 0;
+  const bool narrow = ff * 2 <= sm_count() * 3 * (GEMV_THREADS / 32);
+  if (a.k >= 8192 || (narrow && a.k >= 5632)) launch_gemv_bf16<8, true>(p, a.m, stream);
+  else if (narrow && a.k >= 512) launch_gemv_bf16<2, true>(p, a.m, stream);
+  else launch_gemv_bf16<1, true>(p, a.m, stream);
+  const int rc = launch_check("gemv_swiglu", 1);
   return rc == 0 ? 1 : rc;
 }
 

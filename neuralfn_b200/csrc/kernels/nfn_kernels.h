@@ -70,7 +70,7 @@ typedef struct {
 // x_out = resid + RMS(x) * weight, y = RMS(x_out) * weight_next (1 + w each when centered)
 int nfn_rmsnorm_residual_norm(const void* x, const void* weight, const void* resid, void* x_out, const void* weight_next, void* y, long long rows, int C,
                               float eps, float eps_next, int centered, nfn_stream_t stream);
-int nfn_gemm_swiglu(const void* x, int ldx, const void* b, int ldb, void* c, int ldc, int m, int ff, int k, nfn_stream_t stream);
+int nfn_gemm_swiglu(const void* x, int ldx, const void* b, int ldb, void* c, int ldc, int m, int ff, int k, int resident, nfn_stream_t stream);
 int nfn_gemm_bf16(const nfn_gemm_args* args, nfn_stream_t stream);
 // Grouped contraction for expert weight gradients: C[g] = A[K rows of group g, M]^T . B[same rows, N] for every group in one
 // launch. Both operands MN-major; group_rows = groups + 1 device ints (multiples of 64; padding rows zero); C slices

@@ -359,9 +359,10 @@ def test_gemm_slices_in_a_cluster(kernel_lib, a_mn, b_mn, m, n, k):
     _lib.assert_status_ok("gemm slices")
 
 
-@pytest.mark.parametrize("m,ff,k", [(8191, 1048, 512), (4100, 3000, 1032), (2056, 11272, 520)])
+@pytest.mark.parametrize("m,ff,k", [(8191, 1048, 512), (4100, 3000, 1032), (2056, 11272, 520), (1, 136, 64), (2, 1000, 5640), (1, 5632, 2048), (2, 136, 8200)])
 def test_gemm_swiglu(kernel_lib, m, ff, k):
-    """Gate and up of a column in one pair tile: a last column tile that runs from the gates into the ups, row and k remainders. One rounding to bf16 of
+    """Gate and up of a column in one pair tile: a last column tile that runs from the gates into the ups, row and k remainders;
+    gate and up row of a warp pair for one and two rows, at each number of warps that share it. One rounding to bf16 of
     fp32 values."""
     import ctypes
     from neuralfn_b200.ops import _lib
@@ -369,7 +370,7 @@ def test_gemm_swiglu(kernel_lib, m, ff, k):
     x, w = torch.randn(m, k, device="cuda").bfloat16(), (torch.randn(2 * ff, k, device="cuda") * k ** -0.5).bfloat16()
     out = torch.full((m + 1, ff + 8), 7.0, device="cuda", dtype=torch.bfloat16)
     P, I = ctypes.c_void_p, ctypes.c_int
-    rc = _lib.load().nfn_gemm_swiglu(P(x.data_ptr()), I(k), P(w.data_ptr()), I(k), P(out.data_ptr()), I(ff + 8), I(m), I(ff), I(k), P(_lib.stream_ptr()))
+    rc = _lib.load().nfn_gemm_swiglu(P(x.data_ptr()), I(k), P(w.data_ptr()), I(k), P(out.data_ptr()), I(ff + 8), I(m), I(ff), I(k), I(0), P(_lib.stream_ptr()))
     assert rc == 1
     g, u = (x.double() @ w.double().T).split(ff, -1)
     ref = torch.nn.functional.silu(g) * u

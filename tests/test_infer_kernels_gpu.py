@@ -409,3 +409,33 @@ def test_rmsnorm_residual_norm_equals_the_two_passes(kernel_lib, rows, C, center
     want_y, _, _ = K.norm_forward(res, w2, None, mode=K.NORM_RMS, eps=1e-5, centered=centered)   # of the sum as stored: a step there is not a step here
     for a, b in ((res, want), (y, want_y)):
         assert bool(((a.float() - b.float()).abs() <= 2.0 ** -7 * b.float().abs() + 1e-6).all())
+
+
+@pytest.mark.parametrize("rows,Hq,Hkv,hd,rot", [(1, 1, 1, 64, 64), (37, 5, 3, 64, 64), (513, 32, 8, 128, 128), (7, 3, 1, 128, 48), (5, 2, 2, 64, 16)])
+@pytest.mark.parametrize("convention", ["hf", "legacy"])
+def test_rope_in_vectors_equals_the_element_form(kernel_lib, rows, Hq, Hkv, hd, rot, convention):
+    """Rows on 16-byte boundaries take eight elements per load; a row pitch that is not a multiple of eight the element kernel. The rotation is the same
+    arithmetic (one bf16 step for contracted multiply-adds); the norm's sum of squares is in another order."""
+    from neuralfn_b200.ops import infer
+    torch.manual_seed(rows)
+    H, dev = Hq + Hkv, _dev()
+    src = torch.randn(rows, H * hd + 8, device=dev).bfloat16()
+    cos, sin = infer.rope_tables(700, rot, 10000.0, device=dev)
+    pos = torch.randint(0, 800, (rows,), device=dev, dtype=torch.int32)      # some past the table: clamped
+    qw, kw = (torch.randn(hd, device=dev).bfloat16() for _ in range(2))
+    for norm in (False, True):
+        if norm and rot != hd:
+            continue
+        out = []
+        for pitch in (H * hd + 8, H * hd + 10):
+            x = torch.zeros(rows, pitch, device=dev, dtype=torch.bfloat16)
+            x[:, :H * hd + 8] = src
+            rstd = torch.zeros(rows * H, device=dev)
+            kw_ = dict(T=max(1, rows // 2), n_q_heads=Hq, n_kv_heads=Hkv, head_dim=hd, cos=cos, sin=sin, convention=convention, positions=pos)
+            if norm:
+                infer.qk_norm_rope_forward(x, q_weight=qw, k_weight=kw, q_scale=0.3, rstd=rstd, **kw_)
+            else:
+                infer.rope_inplace(x, rot_dim=rot, q_scale=0.3 if rot == hd else 1.0, **kw_)
+            out.append((x[:, :H * hd + 8].float(), rstd))
+        assert bool(((out[0][0] - out[1][0]).abs() <= 2.0 ** -7 * out[1][0].abs() + 1e-5).all())
+        assert torch.equal(out[0][0][:, H * hd:], src[:, H * hd:].float()) and torch.allclose(out[0][1], out[1][1], rtol=1e-5)

@@ -66,6 +66,8 @@ KERNELS: tuple[KernelEntry, ...] = (
     _k("kv_commit", "nfn_kv_commit_layers"), _k("kv_cache_write", "nfn_kv_cache_write"),
     _k("layernorm / rmsnorm forward", "nfn_norm_forward", ("bf16",), False, "centred scale"),
     _k("norm backward dx", "nfn_norm_backward_dx"), _k("norm backward dw db", "nfn_norm_backward_wb"),
+    _k("gate and up product with SwiGLU", "nfn_gemm_swiglu", ("bf16",), True, "one or two rows, and prompts on CTA pairs"),
+    _k("rmsnorm + residual + next norm", "nfn_rmsnorm_residual_norm"), _k("k-quant products on resident weights", "nfn_kquant_gemv_resident"),
     _k("rmsnorm + residual", "nfn_rmsnorm_residual"), _k("qk_norm", "nfn_qk_norm_forward"), _k("qk_norm backward", "nfn_qk_norm_backward"),
     _k("rope", "nfn_rope_inplace"), _k("qk_norm + rope", "nfn_qk_norm_rope_forward"),
     _k("cross_entropy", "nfn_cross_entropy", ("bf16",), False, "soft-cap derivative, z-loss, in-place gradient"),

@@ -332,10 +332,12 @@ extern "C" int nfn_gemm_bf16(const nfn_gemm_args* args, nfn_stream_t stream_) {
     if (rc != 0) return rc < 0 ? rc : 0;
   }
   const int sms = sm_count();
-  // split-K: only for plain products (no fused element-wise epilogue)
+  // split-K: only for plain products (no fused element-wise epilogue: the slices are summed without one). A number of slices given by the
+  // caller counts where that holds and the workspace takes them; otherwise the product runs whole.
   const int plain_mask = NFN_EPI_BIAS | NFN_EPI_SAVE_PRE | NFN_EPI_RESID | NFN_EPI_DACT | (0xF << NFN_EPI_ACT_SHIFT);
-  const bool may_split = a.split_k != 1 && !(a.flags & plain_mask) && a.workspace;
-  const GemmPlan plan = plan_gemm(a, sms, pair_enabled(), may_split, a.split_k > 1 ? a.split_k : 0);
+  const int given = a.split_k > 1 ? a.split_k : 0;
+  const bool may_split = (given || a.split_k == 0) && !(a.flags & plain_mask) && a.workspace && (long long)given * a.m * a.n * 4 <= a.workspace_bytes;
+  const GemmPlan plan = plan_gemm(a, sms, pair_enabled(), may_split, may_split ? given : 0);
   if (plan.tile == TILE_CLUSTER) return launch_gemm_slices(a, plan.split, stream);
   if (plan.tile == TILE_PAIR) {
     const int rc = launch_gemm_pair(a, plan.split, stream, nullptr, 0, 0);

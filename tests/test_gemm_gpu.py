@@ -377,3 +377,35 @@ def test_gemm_swiglu(kernel_lib, m, ff, k):
     _lib.assert_status_ok("gemm_swiglu")
     assert bool(((out[:m, :ff].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4).all())
     assert bool((out[m:] == 7).all()) and bool((out[:, ff:] == 7).all())
+
+
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
+@pytest.mark.parametrize("m,n,k", [(96, 264, 1032), (264, 520, 4104), (2056, 2312, 1032)])
+@pytest.mark.parametrize("split", [2, 5])
+def test_gemm_with_given_slices_keeps_its_epilogue(kernel_lib, a_mn, b_mn, m, n, k, split):
+    """A number of K slices given together with an epilogue that slices cannot carry: the product runs with that epilogue. Plain, accumulating and
+    scaled products take the slices."""
+    from neuralfn_b200.ops import _lib
+    from neuralfn_b200.ops.gemm import gemm
+    torch.manual_seed(m + split)
+    dev = "cuda"
+    a = torch.randn((k, m) if a_mn else (m, k), device=dev, dtype=torch.bfloat16)
+    b = torch.randn((k, n) if b_mn else (n, k), device=dev, dtype=torch.bfloat16)
+    bias, res = torch.randn(n, device=dev).bfloat16(), torch.randn(m, n, device=dev).bfloat16()
+    s = k ** -0.5
+    base = _ref(a, b, a_mn, b_mn) * s
+    gelu = lambda t: torch.nn.functional.gelu(t, approximate="tanh")  # noqa: E731
+    ws = torch.empty(5 * m * n * 4, device=dev, dtype=torch.uint8)
+    run = lambda **kw: gemm(a, b, a_mn=a_mn, b_mn=b_mn, alpha=s, workspace=ws, split_k=split, **kw)  # noqa: E731
+    _close(run(), base, 64)
+    _close(run(accum=True, out=res.clone()), base + res.float(), 64)
+    _close(run(bias=bias), base + bias.float(), 64)
+    _close(run(resid=res), base + res.float(), 64)
+    _close(run(act="gelu_tanh"), gelu(base), 64)
+    pre = torch.zeros(m, n, device=dev, dtype=torch.bfloat16)
+    _close(run(bias=bias, act="gelu_tanh", save_pre=pre), gelu(base + bias.float()), 64)
+    _close(pre, base + bias.float(), 64)
+    z = res.float().requires_grad_(True)
+    gelu(z).sum().backward()
+    _close(run(act="gelu_tanh", dact_pre=res), base * z.grad, 64)
+    _lib.assert_status_ok("gemm slices with an epilogue")

@@ -197,6 +197,26 @@ def test_component_sources_exist():
         assert len(_build._sources(name)) == len(files)
 
 
+def test_component_sources_define_what_they_call():
+    """A component is a library of its own: an entry point that one of its sources calls, and a function that it declares from another file, has a body
+    in one of its sources. Read from the text of the sources."""
+    import re
+    from neuralfn_b200.ops import _build
+    code = {s.name: re.sub(r"//.*", "", s.read_text()) for s in _build._sources("all")}
+    head = r"^(?:extern \"C\" )?(?!return|else|static|inline)[a-z][\w ]*[ *&]+(\w+)\((?:[^(){};]|\([^()]*\))*\)\s*"
+    defined = {}
+    for name, text in code.items():
+        for function in re.findall(head + r"\{", text, re.M):
+            defined.setdefault(function, set()).add(name)
+    for component in _build.COMPONENTS:
+        sources = {s.name for s in _build._sources(component)}
+        for name in sources:
+            wanted = set(re.findall(r"\b(nfn_\w+)\(", code[name])) & defined.keys() | set(re.findall(head + ";", code[name], re.M))
+            for function in wanted:
+                assert defined[function] & sources, f"{component}: {name} calls {function}, defined in {sorted(defined[function])}"
+    assert "gemm_slices.cu" in defined["launch_gemm_slices"] and "gemm_tcgen05.cu" in defined["nfn_gemm_bf16"]
+
+
 def test_step_entries_are_checked_before_the_engine_sees_them():
     from neuralfn_b200.serving.engine import EngineError, ResidentEngine
     eng = ResidentEngine.__new__(ResidentEngine)

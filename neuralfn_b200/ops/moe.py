@@ -205,6 +205,31 @@ def moe_experts_native_ok(x: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, w
             and d % 64 == 0 and h % 64 == 0 and E <= 256 and indices.shape[-1] <= 8 and x.shape[0] > 0)
 
 
+def _expert_operands(x, w1, w2, w3, weights, indices):
+    """The routing weights as [T, k] and the indices as whole numbers, both on x's device. The kernels get addresses only, so whatever does not fit x and
+    the others is refused here."""
+    if x.dim() != 2 or w1.dim() != 3 or indices.dim() not in (1, 2):
+        raise RuntimeError(f"moe_experts: x {tuple(x.shape)}, w1 {tuple(w1.shape)}, indices {tuple(indices.shape)}: need [T, d], [E, d, h], [T, k]")
+    T, d = x.shape
+    E, _, h = w1.shape
+    k = indices.shape[-1]
+    if tuple(w1.shape) != (E, d, h) or tuple(w3.shape) != (E, d, h) or tuple(w2.shape) != (E, h, d):
+        raise RuntimeError(f"moe_experts: w1 {tuple(w1.shape)}, w3 {tuple(w3.shape)} must be [E, {d}, h], w2 {tuple(w2.shape)} [E, h, {d}]")
+    if indices.numel() != T * k or indices.dtype not in (torch.uint8, torch.int8, torch.int16, torch.int32, torch.int64):
+        raise RuntimeError(f"moe_experts: indices {tuple(indices.shape)} {indices.dtype}: need whole numbers, k for each of {T} tokens")
+    if any(t.dtype != torch.bfloat16 for t in (x, w1, w2, w3)):
+        raise RuntimeError("moe_experts: x, w1, w2 and w3 must be bf16")
+    if any(t.device != x.device for t in (w1, w2, w3)):
+        raise RuntimeError("moe_experts: w1, w2 and w3 must be on the device of x")
+    if weights.shape != (T, k) or weights.device != x.device:
+        weights = weights.to(x.device).expand(T, k)
+    return weights, indices.to(x.device).reshape(T, k)
+
+
 def moe_experts(x: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, w3: torch.Tensor, weights: torch.Tensor, indices: torch.Tensor) -> torch.Tensor:
-    """Differentiable expert FFN on the native kernels (see ``_MoEExpertsFn``)."""
+    """Differentiable expert FFN on the native kernels (see ``_MoEExpertsFn``). ``weights`` of one column, one row or one number are
+    expanded; weights and indices may lie on the host."""
+    weights, indices = _expert_operands(x, w1, w2, w3, weights, indices)
+    if not x.is_cuda:
+        raise RuntimeError("moe_experts: x must be on a CUDA device")
     return _MoEExpertsFn.apply(x.contiguous(), w1, w2, w3, weights, indices)

@@ -110,3 +110,26 @@ def test_moe_experts_refuses_an_expert_that_is_not_there(kernel_lib):
         with pytest.raises(RuntimeError):
             moe_experts(x, w, w, w, wt, torch.tensor([[0], [bad], [1]], device="cuda"))
     moe_experts(x, w, w, w, wt, torch.tensor([[0], [3], [1]], device="cuda"))
+
+
+def _experts_case(T, d, h, E, k, seed, index_dtype=torch.int64):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    t = [r(T, d).bfloat16(), (r(E, d, h) * 0.05).bfloat16(), (r(E, h, d) * 0.05).bfloat16(), (r(E, d, h) * 0.05).bfloat16()]
+    wt, idx = torch.softmax(r(T, E), -1).topk(k, -1)
+    return t, wt, idx.to(index_dtype), r(T, d).bfloat16()
+
+
+def test_moe_experts_takes_weights_and_indices_as_they_come(kernel_lib):
+    """One weight per token, indices of another whole-number type, either of them on the host: the values of the full device tensors."""
+    from neuralfn_b200.ops.moe import moe_experts
+    t, wt, idx, dout = _experts_case(130, 64, 192, 8, 3, 5)
+    one = wt[:, :1].clone().requires_grad_(True)
+    want_in = wt[:, :1].expand(-1, 3).clone().requires_grad_(True)
+    want = moe_experts(*t, want_in, idx)
+    got = moe_experts(*t, one, idx)
+    assert torch.equal(got, want)
+    torch.testing.assert_close(torch.autograd.grad(got, one, dout)[0], torch.autograd.grad(want, want_in, dout)[0].sum(1, keepdim=True))
+    full = moe_experts(*t, wt, idx)
+    for w, i in ((wt, idx.int()), (wt, idx.cpu()), (wt.cpu(), idx), (wt.double(), idx.short())):
+        assert torch.equal(moe_experts(*t, w, i), full)

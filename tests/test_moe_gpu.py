@@ -133,3 +133,37 @@ def test_moe_experts_takes_weights_and_indices_as_they_come(kernel_lib):
     full = moe_experts(*t, wt, idx)
     for w, i in ((wt, idx.int()), (wt, idx.cpu()), (wt.cpu(), idx), (wt.double(), idx.short())):
         assert torch.equal(moe_experts(*t, w, i), full)
+
+
+def _experts_exact(t, wt, idx):
+    x, w1, w2, w3 = (v.double() for v in t)
+    out = torch.zeros_like(x)
+    for e in range(w1.shape[0]):
+        rows, place = (idx == e).nonzero(as_tuple=True)
+        y = (torch.nn.functional.silu(x[rows] @ w1[e]) * (x[rows] @ w3[e])) @ w2[e]
+        out = out.index_add(0, rows, y * wt.double()[rows, place][:, None])
+    return out
+
+
+@pytest.mark.parametrize("T,d,h,E,k", [(50, 72, 40, 4, 2), (33, 64, 72, 3, 1), (40, 136, 64, 6, 3), (129, 64, 64, 16, 9), (7, 64, 128, 32, 32)])
+def test_moe_experts_of_other_widths_and_counts(kernel_lib, T, d, h, E, k):
+    """Widths that are multiples of eight only, more than eight experts per token: within the roundings to bf16 (see above) of the 64-bit values."""
+    from neuralfn_b200.ops.moe import moe_experts
+    t, wt, idx, dout = _experts_case(T, d, h, E, k, T + d)
+    got_in = [v.clone().requires_grad_(True) for v in (*t, wt)]
+    got = moe_experts(*got_in, idx)
+    grads = torch.autograd.grad(got, got_in, dout)
+    ref_in = [v.double().requires_grad_(True) for v in (*t, wt)]
+    out = _experts_exact(ref_in[:4], ref_in[4], idx)
+    want = torch.autograd.grad(out, ref_in, dout.double())
+    for name, a, b in zip(("out", "dx", "dw1", "dw2", "dw3", "dweights"), (got, *grads), (out, *want)):
+        assert float((a.double() - b).norm()) <= 0.012 * float(b.norm()) + 1e-12, name
+
+
+def test_moe_experts_without_tokens(kernel_lib):
+    from neuralfn_b200.ops.moe import moe_experts
+    t, wt, idx, dout = _experts_case(0, 64, 128, 4, 2, 0)
+    got_in = [v.clone().requires_grad_(True) for v in (*t, wt)]
+    got = moe_experts(*got_in, idx)
+    grads = torch.autograd.grad(got, got_in, dout)
+    assert got.shape == (0, 64) and all(a.shape == b.shape and not bool(a.any()) for a, b in zip(grads, got_in))

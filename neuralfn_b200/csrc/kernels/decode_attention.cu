@@ -759,7 +759,14 @@ decode_attention_mma_kernel(const DecodeParams p) {
       const float4 v = __ldcg(reinterpret_cast<const float4*>(ao + (long long)s * (ROWS * HD) + e));
       acc.x += w * v.x; acc.y += w * v.y; acc.z += w * v.z; acc.w += w * v.w;
     }
-    *reinterpret_cast<uint2*>(out + e) = make_uint2(pack_bf16x2(acc.x, acc.y), pack_bf16x2(acc.z, acc.w));
+    if ((reinterpret_cast<uintptr_t>(p.out) & 7) == 0) {
+      *reinterpret_cast<uint2*>(out + e) = make_uint2(pack_bf16x2(acc.x, acc.y), pack_bf16x2(acc.z, acc.w));
+    } else {                                          // the caller's output may start at any element
+      out[e] = __float2bfloat16(acc.x);
+      out[e + 1] = __float2bfloat16(acc.y);
+      out[e + 2] = __float2bfloat16(acc.z);
+      out[e + 3] = __float2bfloat16(acc.w);
+    }
   }
 }
 

@@ -205,6 +205,24 @@ def test_decode_attention_cut_by_length(hd, Hq, Hkv, cap, B):
     assert torch.equal(kc, k_ref) and torch.equal(vc, v_ref) and int(ws.buf[:256].sum()) == 0
 
 
+@pytest.mark.parametrize("offset", [1, 2, 4])
+@pytest.mark.parametrize("length", [40, 1500])
+def test_decode_attention_into_any_element(offset, length):
+    """An output that starts at an element of its own, with one split and with many: the bits of the aligned output and nothing beside it."""
+    from neuralfn_b200.ops import infer
+    torch.manual_seed(length)
+    dev, B, Hq, Hkv, hd, cap = _dev(), 3, 16, 4, 64, 2048
+    kc, vc = (torch.randn(B, Hkv, cap, hd, device=dev).bfloat16() for _ in range(2))
+    qkv, lengths = torch.randn(B, (Hq + 2 * Hkv) * hd, device=dev).bfloat16(), torch.full((B,), length, dtype=torch.int32, device=dev)
+    ws = infer.DecodeAttentionWorkspace(B, Hq, Hkv, hd, dev)
+    kw = dict(n_q_heads=Hq, n_kv_heads=Hkv, head_dim=hd, workspace=ws)
+    want = infer.decode_attention(qkv, kc, vc, lengths, **kw)
+    flat = torch.full((B * Hq * hd + 16,), 7.0, device=dev, dtype=torch.bfloat16)
+    out = flat[offset:offset + B * Hq * hd].view(B, Hq * hd)
+    assert infer.decode_attention(qkv, kc, vc, lengths, out=out, **kw) is out
+    assert torch.equal(out, want) and bool((flat[:offset] == 7).all()) and bool((flat[offset + B * Hq * hd:] == 7).all())
+
+
 @pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K"])
 def test_kquant_dequant_matches_numpy_oracle(name):
     from neuralfn_b200.ops import infer

@@ -79,6 +79,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
     if (static_cast<uint32_t>(smem - smem_raw) + C::SMEM > dyn) {
       if (threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, NFN_ERR_WAIT_MISC);
+      grid_wait();  // no block ends before the launches ahead of this one have
       return;
     }
   }

@@ -6,6 +6,10 @@
 // and the tokens its eight columns. A 4-bit value becomes bf16 by a shift and one logic operation ((q << 3) | 0x4180 is 16 + q
 // exactly), the products of a 32-weight group are summed unscaled, and scale and offset enter once per group in fp32:
 //   y += (d s) * sum (16 + q) x  -  (16 d s + dmin m) * sum x
+// The two parts of a group carry 16 sum x, which cancels in fp32: against sums over decoded weights that is at most a few more roundings of 16 times
+// the offset's size (the error against 64 bits is the output's rounding to bf16 in both kernels, 1.66e-3). Where an activation is
+// infinite, undefined or beyond 2^65 the parts would cancel to nothing or overflow, so a token with such a value in a warp's part of K gets that part
+// summed over decoded weights, one by one.
 // The contraction index is permuted so that a lane's 8 bytes of a group are its operands as they lie; the tokens are put into
 // that order in shared memory once per CTA, with the sums of their groups.
 //
@@ -116,6 +120,32 @@ __device__ __forceinline__ void q4_multiply(const Q4Block& v, const uint4* xs, c
   chunk(integral_constant<int, 6>{}, integral_constant<int, 7>{}, v.q[0][3], v.q[1][3]);
 }
 
+// The larger magnitudes of two pairs (undefined if one is), and whether either value is infinite, undefined or at least 2^65: an exponent field
+// of 192 and above
+__device__ __forceinline__ __nv_bfloat162 q4_top(__nv_bfloat162 a, uint32_t w) { return __hmax2_nan(a, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w))); }
+__device__ __forceinline__ bool q4_beyond(__nv_bfloat162 a) {
+  const uint32_t w = *reinterpret_cast<const uint32_t*>(&a);
+  return w & (w << 1) & 0x40004000u;
+}
+
+// sum over blocks k_lo .. k_hi - 1 of one weight row times one token, weight by weight. A call of its own: the kernel has no registers to
+// spare (looking for such values and this branch cost 1 % of its time, with the sum in place 2 %).
+__device__ __noinline__ float q4_sum_decoded(const uint8_t* row, const __nv_bfloat16* x, int k_lo, int k_hi) {
+  float acc = 0.f;
+  for (int kb = k_lo; kb < k_hi; ++kb) {
+    const uint8_t* blk = row + (size_t)kb * Q4_BLOCK;
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(blk));
+    for (int i = 0; i < 256; ++i) {
+      const int s = i >> 5, byte = blk[16 + 32 * (s >> 1) + (i & 31)];
+      const uint8_t* q = blk + 4;
+      const int sc = s < 4 ? q[s] & 63 : (q[s + 4] & 15) | ((q[s - 4] >> 6) << 4), mn = s < 4 ? q[s + 4] & 63 : (q[s + 4] >> 4) | ((q[s] >> 6) << 4);
+      const float w = f.x * (float)sc * (float)(s & 1 ? byte >> 4 : byte & 15) - f.y * (float)mn;
+      acc = fmaf(w, __bfloat162float(x[kb * 256 + i]), acc);
+    }
+  }
+  return acc;
+}
+
 __global__ void __launch_bounds__(Q4_THREADS, 2)
 gemv_q4k_kernel(const Q4Params p) {
   extern __shared__ __align__(128) unsigned char q4_smem[];
@@ -140,6 +170,7 @@ gemv_q4k_kernel(const Q4Params p) {
   if (busy && !p.static_w) q4_load(cur, r0, r1, k_lo, j);
 
   // this warp's share of the tokens: pairs (0, 2), (1, 3), (4, 6), (5, 7) of every run of eight
+  __nv_bfloat162 top = __floats2bfloat162_rn(0.f, 0.f);
 #pragma unroll 4
   for (int i = k_lo * 8; i < k_hi * 8; ++i) {                                       // groups of 32
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
@@ -150,7 +181,9 @@ gemv_q4k_kernel(const Q4Params p) {
     s += __shfl_xor_sync(0xffffffffu, s, 2);
     xs[i * 32 + lane] = make_uint4(__byte_perm(v.x, v.y, 0x5410), __byte_perm(v.x, v.y, 0x7632), __byte_perm(v.z, v.w, 0x5410), __byte_perm(v.z, v.w, 0x7632));
     if (j == 0) sums[i * 8 + g] = s;
+    top = q4_top(q4_top(q4_top(q4_top(top, v.x), v.y), v.z), v.w);
   }
+  const unsigned beyond_of = __ballot_sync(0xffffffffu, q4_beyond(top));              // bits 4 g .. 4 g + 3: token g
   __syncwarp();
 
   for (int it = 0; tile < p.tiles; ++it) {
@@ -163,6 +196,15 @@ gemv_q4k_kernel(const Q4Params p) {
       if (kb + 1 < k_hi) q4_load(cur, r0, r1, kb + 1, j);
       else if (next < p.tiles) q4_load(cur, n0, n1, k_lo, j);
       q4_multiply(v, xs + (size_t)kb * 256, reinterpret_cast<const float2*>(sums + (size_t)kb * 64), lane, acc);
+    }
+    if (beyond_of) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (!((beyond_of >> (4 * (2 * j + h))) & 15u)) continue;
+        const __nv_bfloat16* x = p.x + (size_t)(2 * j + h) * p.ldx;
+        acc[h] = q4_sum_decoded(r0, x, k_lo, k_hi);
+        acc[2 + h] = q4_sum_decoded(r1, x, k_lo, k_hi);
+      }
     }
     float* mine = part + ((it & 1) * Q4_WARPS + warp) * 128;
     *reinterpret_cast<float2*>(mine + g * 8 + 2 * j) = make_float2(acc[0], acc[1]);

@@ -281,6 +281,30 @@ def test_q4k_gemv_against_64_bit(B, N, K):
     assert bool(((got.double() - ref).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("B,N,K", [(1, 16, 256), (4, 37, 2048), (8, 130, 4096)])
+def test_q4k_gemv_of_infinities_and_huge_values(B, N, K):
+    """An infinite, undefined or huge activation gives what the sum over the decoded weights gives, and the other token rows the bits they have
+    without it."""
+    from neuralfn_b200.ops import infer
+    from neuralfn_b200.quant import kquant
+    t, dev = kquant.GGML_TYPE["Q4_K"], _dev()
+    raw = kquant.random_blocks(t, N * K // 256, seed=N)
+    w = torch.from_numpy(kquant.dequantize(t, raw.tobytes())).view(N, K).to(dev)
+    packed, clean = torch.from_numpy(raw).to(dev).reshape(-1), torch.randn(B, K, device=dev).bfloat16()
+    before = infer.kquant_gemv(t, packed, clean, N)
+    for row, col, v in ((0, 0, math.inf), (B - 1, K - 1, -math.inf), (B // 2, K // 2 + 3, math.nan), (0, 37, 2.0 ** 120), (B - 1, 100, -2.0 ** 66)):
+        x = clean.clone()
+        x[row, col] = v
+        got = infer.kquant_gemv(t, packed, x, N).float()
+        ref = x[row].double() @ w.double().T
+        if math.isfinite(v):
+            assert bool(((got[row].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * (x[row].double().abs() @ w.double().abs().T)).all())
+        else:
+            assert torch.equal(got[row].nan_to_num(nan=7.0), ref.float().nan_to_num(nan=7.0))
+        others = [b for b in range(B) if b != row]
+        assert torch.equal(got[others], before.float()[others])
+
+
 def _block_attention_ref(qkv, kc, vc, lengths, rows, Hq, Hkv, D, window, causal, n_rows):
     """fp32 oracle: logical key list per sequence = cached positions still in the cache + block rows."""
     B, _, cap, _ = kc.shape

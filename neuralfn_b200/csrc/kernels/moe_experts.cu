@@ -535,11 +535,13 @@ extern "C" int nfn_moe_experts_forward(const nfn_moe_experts_args* args, nfn_str
   cudaGetDevice(&dev);
   static thread_local BadIndex bad_of[64];
   BadIndex& bad = bad_of[dev & 63];
-  if (!bad.ready()) return launch_check("moe_experts setup", 0);
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   cudaStreamIsCapturing(stream, &capture);
   const bool eager = capture == cudaStreamCaptureStatusNone;
-  if (eager) *bad.host = 0;
+  if (eager) {
+    if (!bad.ready()) return launch_check("moe_experts setup", 0);   // allocates: not during a capture, which has no use for it
+    *bad.host = 0;
+  }
 
   const int n = a.tokens * a.top, blocks = ceil_div(n, MX_IDX);
   const long long pad = (long long)a.experts * (MX_TILE - 1);

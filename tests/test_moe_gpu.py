@@ -167,3 +167,46 @@ def test_moe_experts_without_tokens(kernel_lib):
     got = moe_experts(*got_in, idx)
     grads = torch.autograd.grad(got, got_in, dout)
     assert got.shape == (0, 64) and all(a.shape == b.shape and not bool(a.any()) for a, b in zip(grads, got_in))
+
+
+def test_moe_experts_in_a_graph(kernel_lib):
+    """Captured forward and backward on a thread whose first expert call this is, replayed on other inputs: the values of the eager call. An expert that is
+    not there leaves its entry out of the replay."""
+    import threading
+    from neuralfn_b200.ops.moe import moe_experts
+    t, wt, idx, dout = _experts_case(300, 64, 128, 8, 2, 1)
+    t2, wt2, idx2, _ = _experts_case(300, 64, 128, 8, 2, 2)
+    leaves = [v.requires_grad_(True) for v in (*t, wt)]
+    moe_experts(*leaves, idx)                                       # kernels loaded, attributes set
+    torch.cuda.synchronize()
+    got, failed = [], []
+
+    def capture():
+        try:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                out = moe_experts(*leaves, idx)
+                grads = torch.autograd.grad(out, leaves, dout)
+            got.extend([graph, out, *grads])
+        except Exception as e:  # noqa: BLE001
+            failed.append(e)
+
+    worker = threading.Thread(target=capture)
+    worker.start()
+    worker.join()
+    assert not failed, failed
+    graph, *results = got
+    with torch.no_grad():
+        for a, b in zip((*leaves, idx), (*t2, wt2, idx2)):
+            a.copy_(b)
+    graph.replay()
+    torch.cuda.synchronize()
+    eager = moe_experts(*leaves, idx)
+    for a, b in zip(results, (eager, *torch.autograd.grad(eager, leaves, dout))):
+        assert torch.equal(a, b)
+    with torch.no_grad():
+        idx[5, 1] = 99
+    graph.replay()
+    torch.cuda.synchronize()
+    alone = _experts_exact([v[5:6] if i == 0 else v for i, v in enumerate(leaves[:4])], leaves[4][5:6, :1], idx[5:6, :1])
+    assert float((results[0][5].double() - alone[0]).norm()) <= 0.012 * float(alone.norm())

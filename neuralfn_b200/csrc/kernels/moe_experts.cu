@@ -480,6 +480,8 @@ static int check_args(const nfn_moe_experts_args* a) {
        reinterpret_cast<uintptr_t>(a->work) | reinterpret_cast<uintptr_t>(a->out) | reinterpret_cast<uintptr_t>(a->dout) | reinterpret_cast<uintptr_t>(a->dx) |
        reinterpret_cast<uintptr_t>(a->dw1) | reinterpret_cast<uintptr_t>(a->dw2) | reinterpret_cast<uintptr_t>(a->dw3) | reinterpret_cast<uintptr_t>(a->scratch)) & 15)
     return fail(-1, "moe_experts: operands must be 16-byte aligned");
+  if ((reinterpret_cast<uintptr_t>(a->work) | reinterpret_cast<uintptr_t>(a->scratch)) & 31)
+    return fail(-1, "moe_experts: work and scratch must be 32-byte aligned");   // the products' epilogues store 32 bytes at a time
   return 0;
 }
 

@@ -685,7 +685,8 @@ int nfn_moe_rows(const nfn_moe_rows_args* args, nfn_stream_t stream);
 // ---- expert feed-forward with gradients (moe_experts.cu) ----------------------------------------------------------------------
 // out[t] = sum_j weights[t][j] * (silu(x[t] w1[e]) * (x[t] w3[e])) w2[e], e = indices[t][j]; w1, w3 [experts][d][ff], w2 [experts][ff][d], all bf16 and
 // contiguous, weights fp32. top <= 8, experts <= 256, d and ff multiples of 64. capacity_rows: tokens * top + 127 * experts, up to a whole 128.
-// work: nfn_moe_experts_work_bytes, kept from the forward to the backward call (save = 1); scratch: nfn_moe_experts_scratch_bytes, backward only.
+// work: nfn_moe_experts_work_bytes, kept from the forward to the backward call (save = 1); scratch: nfn_moe_experts_scratch_bytes, backward only; both
+// 32-byte aligned, the other operands 16.
 // The forward call refuses an index outside [0, experts); under stream capture such entries are left out instead.
 typedef struct {
   const void* x; const void* w1; const void* w2; const void* w3;

@@ -48,3 +48,16 @@ def test_moe_experts_refuses_host_tensors(monkeypatch):
 def test_expert_operands_expands_weights(weights):
     full, indices = moe._expert_operands(**{**_operands(), "weights": weights, "indices": torch.zeros(6, 2, dtype=torch.int32)})
     assert full.shape == (6, 2) and indices.shape == (6, 2)
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="addresses that must never reach a device")
+@pytest.mark.parametrize("name,entry", [("work", "forward"), ("work", "backward"), ("scratch", "backward")])
+def test_workspaces_off_32_bytes_are_refused_before_a_launch(name, entry):
+    """The epilogues store 32 bytes at a time. Addresses that are never read: the check is the first thing the entry does."""
+    import ctypes
+    lib = _lib.load()
+    where = {n: 1 << 20 for n in ("x", "w1", "w2", "w3", "weights", "indices", "out", "work", "dout", "scratch", "dx", "dw1", "dw2", "dw3", "dweights")}
+    where[name] += 16
+    args = moe._ExpertsArgs(**where, tokens=6, d=64, ff=128, experts=4, top=2, capacity_rows=640, save=1)
+    assert getattr(lib, f"nfn_moe_experts_{entry}")(ctypes.byref(args), None) == -1
+    assert b"32-byte aligned" in lib.nfn_last_error()

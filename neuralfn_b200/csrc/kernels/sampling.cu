@@ -233,20 +233,23 @@ sample_rows_kernel(const T* logits, long long ld, int V, int rows, int* out_idx,
     }
   };
   // One block per row and a greedy choice is this pass alone: with element loads it is a chain of V / 1024 latencies
-  // (13 us at 32000). bf16 rows on 16-byte boundaries take eight values per load.
+  // (13 us at 32000). Rows on 16-byte boundaries take 16 bytes per load.
   int tail = 0;
-  if constexpr (sizeof(T) == 2) {
-    if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
-      tail = V & ~7;
+  if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+    constexpr int VEC = 16 / sizeof(T);
+    tail = V & ~(VEC - 1);
 #pragma unroll 4
-      for (int i = threadIdx.x * 8; i < tail; i += 8192) {
-        const uint4 u = ld_after_wait16(p + i);
-        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+    for (int i = threadIdx.x * VEC; i < tail; i += 1024 * VEC) {
+      const uint4 u = ld_after_wait16(p + i);
+      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
+      for (int h = 0; h < 4; ++h) {
+        if constexpr (VEC == 8) {
           const float2 f = unpack_bf16x2(w[h]);
           take(f.x, i + 2 * h);
           take(f.y, i + 2 * h + 1);
+        } else {
+          take(__uint_as_float(w[h]), i + h);
         }
       }
     }

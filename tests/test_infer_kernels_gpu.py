@@ -78,6 +78,24 @@ def test_argmax_rows_ties_and_offsets(dtype):
     assert int(one[0]) == int(logits[0, :1000].float().argmax())
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("V,ld", [(1, 8), (7, 8), (4099, 4104), (8191, 8192), (8200, 8200), (33000, 33001)])
+def test_greedy_rows_of_every_length_and_alignment(dtype, V, ld):
+    """Rows on 16-byte boundaries and off them, tails of a load: the first of equal maxima, undefined values left out, whatever lies behind the row ignored."""
+    from neuralfn_b200.ops import infer
+    g = torch.Generator(device="cuda").manual_seed(V)
+    wide = (torch.randn(5, ld, device=_dev(), generator=g) * 4).to(dtype)
+    wide[:, V:] = 100.0
+    rows = wide[:, :V]
+    rows[1] = -7.0
+    rows[2, V // 2:] = 50.0
+    rows[3, V - 1] = 60.0
+    rows[4, :V // 3] = math.nan
+    want = rows.float().nan_to_num(nan=-math.inf)
+    want = torch.stack([(r == r.max()).nonzero()[0, 0] for r in want])
+    assert torch.equal(infer.sample_rows(rows, temperature=0.0).long(), want)
+
+
 def test_sampling_truncation_and_distribution():
     from neuralfn_b200.ops import infer
     torch.manual_seed(3)

@@ -232,7 +232,26 @@ static GemmPlan plan_gemm(const nfn_gemm_args& a, int sms, bool pairs, bool may_
   return best;
 }
 
+static GemmPlan plan_of(const nfn_gemm_args& a) {
+  // split-K: only for plain products (no fused element-wise epilogue: the slices are summed without one). A number of slices given by the
+  // caller counts where that holds and the workspace takes them; otherwise the product runs whole.
+  const int plain_mask = NFN_EPI_BIAS | NFN_EPI_SAVE_PRE | NFN_EPI_RESID | NFN_EPI_DACT | (0xF << NFN_EPI_ACT_SHIFT);
+  const int given = a.split_k > 1 ? a.split_k : 0;
+  const bool may_split = (given || a.split_k == 0) && !(a.flags & plain_mask) && a.workspace && (long long)given * a.m * a.n * 4 <= a.workspace_bytes;
+  return plan_gemm(a, sm_count(), pair_enabled(), may_split, may_split ? given : 0);
+}
+
 }  // namespace nfn
+
+// The tile shape of a product that goes to the tcgen05 kernels (0: 128 x 128, 1: 128 x 256, 2: 256 x 256 on a CTA pair, 3: a cluster over K) and its
+// slices of K; nothing is launched.
+extern "C" int nfn_gemm_plan(const nfn_gemm_args* args, int* slices) {
+  using namespace nfn;
+  if (!args || !slices || args->m <= 0 || args->n <= 0 || args->k <= 0) return fail(-1, "gemm_plan: bad arguments");
+  const GemmPlan plan = plan_of(*args);
+  *slices = plan.split;
+  return plan.tile;
+}
 
 // 1 (default): products with at most two rows go to the streaming GEMV kernel; 0: always the tensor-core path.
 extern "C" int nfn_gemm_set_gemv_mode(int on) {
@@ -331,13 +350,7 @@ extern "C" int nfn_gemm_bf16(const nfn_gemm_args* args, nfn_stream_t stream_) {
     const int rc = try_launch_skinny(a, stream);
     if (rc != 0) return rc < 0 ? rc : 0;
   }
-  const int sms = sm_count();
-  // split-K: only for plain products (no fused element-wise epilogue: the slices are summed without one). A number of slices given by the
-  // caller counts where that holds and the workspace takes them; otherwise the product runs whole.
-  const int plain_mask = NFN_EPI_BIAS | NFN_EPI_SAVE_PRE | NFN_EPI_RESID | NFN_EPI_DACT | (0xF << NFN_EPI_ACT_SHIFT);
-  const int given = a.split_k > 1 ? a.split_k : 0;
-  const bool may_split = (given || a.split_k == 0) && !(a.flags & plain_mask) && a.workspace && (long long)given * a.m * a.n * 4 <= a.workspace_bytes;
-  const GemmPlan plan = plan_gemm(a, sms, pair_enabled(), may_split, may_split ? given : 0);
+  const GemmPlan plan = plan_of(a);
   if (plan.tile == TILE_CLUSTER) return launch_gemm_slices(a, plan.split, stream);
   if (plan.tile == TILE_PAIR) {
     const int rc = launch_gemm_pair(a, plan.split, stream, nullptr, 0, 0);

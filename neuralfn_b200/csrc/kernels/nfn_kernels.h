@@ -72,6 +72,7 @@ int nfn_rmsnorm_residual_norm(const void* x, const void* weight, const void* res
                               float eps, float eps_next, int centered, nfn_stream_t stream);
 int nfn_gemm_swiglu(const void* x, int ldx, const void* b, int ldb, void* c, int ldc, int m, int ff, int k, int resident, nfn_stream_t stream);
 int nfn_gemm_bf16(const nfn_gemm_args* args, nfn_stream_t stream);
+int nfn_gemm_plan(const nfn_gemm_args* args, int* slices);
 // Grouped contraction for expert weight gradients: C[g] = A[K rows of group g, M]^T . B[same rows, N] for every group in one
 // launch. Both operands MN-major; group_rows = groups + 1 device ints (multiples of 64; padding rows zero); C slices
 // group_stride elements apart. Only alpha, fp32 output and accumulate of the epilogue flags apply.

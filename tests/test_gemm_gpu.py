@@ -23,6 +23,16 @@ def _close(out, ref, k):
     assert fro <= 4e-3, f"relative Frobenius error {fro}"
 
 
+def _route(m, n, k, a_mn, b_mn, split=1, workspace=0):
+    """(tile shape, slices of K) that a plain product takes; no operand is looked at."""
+    import ctypes
+    from neuralfn_b200.ops import _lib
+    a, slices = _lib.GemmArgs(), ctypes.c_int()
+    a.m, a.n, a.k, a.lda, a.ldb, a.ldc = m, n, k, m if a_mn else k, n if b_mn else k, n
+    a.a_mn, a.b_mn, a.alpha, a.split_k, a.workspace, a.workspace_bytes = int(a_mn), int(b_mn), 1.0, split, 256 if workspace else None, workspace
+    return ("128", "256", "pair", "cluster")[_lib.load().nfn_gemm_plan(ctypes.byref(a), ctypes.byref(slices))], slices.value
+
+
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
 @pytest.mark.parametrize("m,n,k", [(128, 128, 64), (256, 256, 128), (384, 768, 768), (1000, 264, 200),
                                    (4096, 2304, 768), (2048, 50304, 768)])
@@ -311,11 +321,16 @@ def test_grouped_contraction_gives_every_experts_weight_gradient(kernel_lib, m, 
 
 
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
-@pytest.mark.parametrize("m,n,k,split", [(2056, 2312, 72, 1), (6664, 776, 1000, 1), (264, 520, 4104, 5), (776, 264, 16392, 0), (136, 19208, 520, 1)])
-def test_gemm_pairs_and_slices_at_edges(kernel_lib, a_mn, b_mn, m, n, k, split):
-    """Remainders of the 256 x 256 pair tile and of the k-block, an uneven last slice, in all four operand layouts; equal results on every run."""
+@pytest.mark.parametrize("m,n,k,split,route", [
+    (2056, 2312, 72, 1, ("128", 1)), (6664, 776, 1000, 1, ("pair", 1)), (264, 520, 4104, 5, ("128", 5)), (776, 264, 16392, 0, ("cluster", 6)),
+    (136, 19208, 520, 1, ("pair", 1)), (1032, 1288, 8200, 0, ("pair", 2)), (2056, 2312, 4104, 2, ("pair", 2)), (776, 1288, 16392, 0, ("pair", 3)),
+    (520, 2056, 8200, 0, ("256", 3)), (4104, 1032, 1000, 5, ("pair", 1))])
+def test_gemm_pairs_and_slices_at_edges(kernel_lib, a_mn, b_mn, m, n, k, split, route):
+    """Remainders of every tile shape and of the k-block, an uneven last slice, slices on CTA pairs, slices that the
+    workspace does not hold, in all four operand layouts; equal results on every run."""
     from neuralfn_b200.ops import _lib
     from neuralfn_b200.ops.gemm import gemm
+    assert _route(m, n, k, a_mn, b_mn, split=split, workspace=64 << 20) == route
     torch.manual_seed(m)
     a = torch.randn((k, m) if a_mn else (m, k), device="cuda", dtype=torch.bfloat16)
     b = torch.randn((k, n) if b_mn else (n, k), device="cuda", dtype=torch.bfloat16)
@@ -329,11 +344,16 @@ def test_gemm_pairs_and_slices_at_edges(kernel_lib, a_mn, b_mn, m, n, k, split):
 
 
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
-@pytest.mark.parametrize("m,n,k", [(136, 128, 520), (256, 264, 1032), (24, 2056, 4104), (520, 136, 6000)])
+@pytest.mark.parametrize("m,n,k", [(136, 128, 520), (256, 264, 1032), (24, 2056, 4104), (520, 136, 6000), (136, 128, 2056), (130, 136, 4104)])
 def test_gemm_slices_in_a_cluster(kernel_lib, a_mn, b_mn, m, n, k):
-    """Fewer tiles than SMs: K cut over a cluster (uneven slices, remainders of tile and k-block, fewer rows than ranks have shares), with every epilogue."""
+    """Fewer tiles than SMs: K cut over a cluster (uneven slices, remainders of tile and k-block, two rows of a tile for more ranks), with every epilogue;
+    the first shape has too short a K and takes whole tiles."""
     from neuralfn_b200.ops import _lib
     from neuralfn_b200.ops.gemm import gemm
+    if a_mn and m % 8:
+        pytest.skip("MN-major A needs M % 8 == 0")
+    tile, slices = _route(m, n, k, a_mn, b_mn)
+    assert tile == ("128" if k < 1000 else "cluster") and (m != 130 or slices > m % 128)
     torch.manual_seed(m)
     dev = "cuda"
     a = torch.randn((k, m) if a_mn else (m, k), device=dev, dtype=torch.bfloat16)

@@ -200,7 +200,7 @@ def test_decode_attention_append_and_attend(hd, Hq, Hkv, cap, ring, decode_impl)
 
 @pytest.mark.parametrize("hd,Hq,Hkv,cap,B", [(128, 16, 4, 2048, 1), (64, 8, 8, 2048, 3), (128, 32, 4, 1500, 40), (64, 48, 4, 1024, 6), (128, 8, 8, 20000, 2)])
 def test_decode_attention_cut_by_length(hd, Hq, Hkv, cap, B):
-    """Lengths around the ends of a step (16), a split (64 to 256 positions) and the cache, one split and many in one launch, sequences left out."""
+    """Lengths around the ends of a step (16), a split (64 to 512 positions) and the cache, one split and many in one launch, sequences left out."""
     from neuralfn_b200.ops import infer
     torch.manual_seed(Hq + cap)
     dev = _dev()

@@ -3,8 +3,9 @@
 //
 // Either operand may be K-major or MN-major, which gives the forward (X W^T),
 // input-gradient (dY W) and weight-gradient (dY^T X) products without any transpose
-// in memory. Weight-gradient shapes (small M x N output, very long K) are split along
-// K into fp32 partial slices that a second small kernel sums.
+// in memory. Products with few tiles are cut along K: over a thread-block cluster that adds its
+// parts on chip (gemm_slices.cu), or, where K is long for the output, into fp32 slices of the
+// workspace that a second small kernel sums.
 //
 // Covers the role of the reference's linear kernels and library GEMM call sites
 // (neuralfn/csrc/tile_cuda/kernels.cu:16746-17574 and its cuBLASLt wrappers) with

@@ -1,11 +1,9 @@
-// Products with one or two rows (single-stream decode: the "matrix" A is one or two token
-// vectors; from three rows on the tensor-core path is faster): C[M, N] = A[M, K] . B[N, K]^T with the GEMM family's epilogue. Such a product only
-// streams the weight matrix once, so it is a pure HBM-bandwidth problem and a tensor-core tile
-// (64 or 128 rows at least) has nothing to contribute: every warp takes one weight row at a
-// time, its 32 lanes read the rows as 16-byte chunks (eight in flight per lane) with streaming
-// loads, multiply with the matching chunks of the token vectors (which stay in L1), and reduce
-// with shuffles. Epilogue order as in the tcgen05 kernels: alpha, bias, activation, residual,
-// accumulate.
+// Products with one or two rows (single-stream decode: the "matrix" A is one or two token vectors; from three rows on the tensor-core
+// path is faster): C[M, N] = A[M, K] . B[N, K]^T with the GEMM family's epilogue. Such a product only streams the weight matrix once, so it is a
+// pure HBM-bandwidth problem and a tensor-core tile (64 or 128 rows at least) has nothing to contribute: one, two or eight warps take a pair of weight
+// rows at a time, their lanes read both rows as 16-byte chunks (eight in flight per lane) with streaming loads, multiply with the matching
+// chunks of the token vectors (which stay in L1), and reduce with shuffles and, for several warps, through shared memory. Epilogue order as
+// in the tcgen05 kernels: alpha, bias, activation, residual, accumulate. In the gated form the pair is a gate row and its up row.
 //
 // Counterpart in the reference: the decode-time `linear_*` kernels of kernels.cu:16746-16840
 // (one thread-tile per output element).
@@ -161,6 +159,22 @@ static void launch_gemv_bf16(const GemvParams& p, int m, cudaStream_t stream) {
   else launch_overlapped(gemv_bf16_kernel<2, KS, GATED>, grid, GEMV_THREADS, 0, stream, p);
 }
 
+// Warps per row pair. Resident weights, us for the product and the one-row norm ahead of it with 1 / 2 / 8 warps:
+//  two, where two for every pair are still one round of all resident warps (the loads of a narrow matrix are then on their way at once) and K is
+//     below 5632: 2048 x 2048 5.9 / 4.2 / 6.0, 3072 x 4096 9.9 / 7.8 / 9.3
+//  eight, there from K = 5632 on: two rows of 2048 x 5632 16.9 / 10.9 / 9.8, one row of 512 11.5 / 7.9 / 5.0, of 2048 level (12.4 / 9.0 / 9.3), of
+//     3072 behind two (12.9 / 9.9 / 11.4)
+//  eight from K = 8192 on for wider ones: 4096 x 8192 18.9 / 19.2 / 16.8, two rows 27.1 / 22.6 / 17.4
+//  one otherwise, the sum over warps costs more than it gives: 11264 x 2048 11.8 / 12.5 / 19.8
+// The lines are rough: eight would be ahead from K = 1024 on at 512 columns, from 4096 on for two rows of 2048 (8.6 / 8.2) and of 4096 (14.8 / 11.9).
+template <bool GATED>
+static void launch_gemv_pairs(const GemvParams& p, int m, cudaStream_t stream) {
+  const bool narrow = (GATED ? p.n : (p.n + 1) / 2) * 2 <= sm_count() * 3 * (GEMV_THREADS / 32);
+  if (p.k >= 8192 || (narrow && p.k >= 5632)) launch_gemv_bf16<8, GATED>(p, m, stream);
+  else if (narrow && p.k >= 512) launch_gemv_bf16<2, GATED>(p, m, stream);
+  else launch_gemv_bf16<1, GATED>(p, m, stream);
+}
+
 // Returns 1 when it launched, 0 when the product is not a GEMV case (the caller continues with the
 // tensor-core path), negative on a launch error.
 int try_launch_gemv(const nfn_gemm_args& a, cudaStream_t stream) {
@@ -180,19 +194,12 @@ int try_launch_gemv(const nfn_gemm_args& a, cudaStream_t stream) {
   p.accum = (a.flags & NFN_EPI_ACCUM) ? 1 : 0;
   p.alpha = a.alpha; p.act_param = a.act_param;
   p.static_b = (a.flags & NFN_GEMM_STATIC_B) ? 1 : 0;
-  // Warps per row pair. Two where that still is one round of all resident warps: the loads of a narrow matrix are then on their way
-  // at once (3072 x 2048, one row: 4.8 us with one, 3.3 with two, 4.2 with four). Eight for long K, where one warp would come back for
-  // the next eight loads five times or more (4096 x 14336: 25.3, 25.1, 24.7, 23.1 us; two rows 35.9 and 24.5; 2048 x 5632, two rows:
-  // 12.9, 7.9, 9.4, 7.1). One otherwise: the sum over warps costs more than it gives (11264 x 2048: 10.4, 10.9, 12.9, 18.3).
-  const bool narrow = (a.n + 1) / 2 * 2 <= sm_count() * 3 * (GEMV_THREADS / 32);
-  if (a.k >= 8192 || (narrow && a.k >= 5632)) launch_gemv_bf16<8>(p, a.m, stream);
-  else if (narrow && a.k >= 512) launch_gemv_bf16<2>(p, a.m, stream);
-  else launch_gemv_bf16<1>(p, a.m, stream);
+  launch_gemv_pairs<false>(p, a.m, stream);
   const int rc = launch_check("gemv_bf16", 1);
   return rc == 0 ? 1 : rc;
 }
 
-// c [m, ff] = silu(a wg^T) * (a wu^T), b = [wg; wu], m <= 2; the warps per row pair as for a product of 2 ff columns.
+// c [m, ff] = silu(a wg^T) * (a wu^T), b = [wg; wu], m <= 2; a pair is a gate row and its up row.
 int launch_gemv_swiglu(const nfn_gemm_args& a, int ff, cudaStream_t stream) {
   GemvParams p{};
   p.a = static_cast<const __nv_bfloat16*>(a.a);
@@ -201,10 +208,7 @@ int launch_gemv_swiglu(const nfn_gemm_args& a, int ff, cudaStream_t stream) {
   p.n = ff; p.k = a.k; p.lda = a.lda; p.ldb = a.ldb; p.ldc = a.ldc;
   p.alpha = 1.f;
   p.static_b = (a.flags & NFN_GEMM_STATIC_B) ? 1 : 0;
-  const bool narrow = ff * 2 <= sm_count() * 3 * (GEMV_THREADS / 32);
-  if (a.k >= 8192 || (narrow && a.k >= 5632)) launch_gemv_bf16<8, true>(p, a.m, stream);
-  else if (narrow && a.k >= 512) launch_gemv_bf16<2, true>(p, a.m, stream);
-  else launch_gemv_bf16<1, true>(p, a.m, stream);
+  launch_gemv_pairs<true>(p, a.m, stream);
   const int rc = launch_check("gemv_swiglu", 1);
   return rc == 0 ? 1 : rc;
 }

@@ -266,25 +266,32 @@ def moe_experts_native_ok(x: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, w
             and d % 64 == 0 and h % 64 == 0 and E <= 256 and indices.shape[-1] <= 8 and x.shape[0] > 0)
 
 
+_WHOLE = frozenset((torch.uint8, torch.int8, torch.int16, torch.int32, torch.int64))
+
+
 def _expert_operands(x, w1, w2, w3, weights, indices):
     """The routing weights as [T, k] and the indices as whole numbers, both on x's device. The kernels get addresses only, so whatever does not fit x and
-    the others is refused here."""
-    if x.dim() != 2 or w1.dim() != 3 or indices.dim() not in (1, 2):
-        raise RuntimeError(f"moe_experts: x {tuple(x.shape)}, w1 {tuple(w1.shape)}, indices {tuple(indices.shape)}: need [T, d], [E, d, h], [T, k]")
-    T, d = x.shape
-    E, _, h = w1.shape
-    k = indices.shape[-1]
-    if tuple(w1.shape) != (E, d, h) or tuple(w3.shape) != (E, d, h) or tuple(w2.shape) != (E, h, d):
-        raise RuntimeError(f"moe_experts: w1 {tuple(w1.shape)}, w3 {tuple(w3.shape)} must be [E, {d}, h], w2 {tuple(w2.shape)} [E, h, {d}]")
-    if indices.numel() != T * k or indices.dtype not in (torch.uint8, torch.int8, torch.int16, torch.int32, torch.int64):
-        raise RuntimeError(f"moe_experts: indices {tuple(indices.shape)} {indices.dtype}: need whole numbers, k for each of {T} tokens")
-    if any(t.dtype != torch.bfloat16 for t in (x, w1, w2, w3)):
+    the others is refused here. Operands that lie as the kernels want them make no call into torch but reads of their fields: a short batch is bound by
+    what the host does."""
+    sx, s1, si = x.shape, w1.shape, indices.shape
+    if len(sx) != 2 or len(s1) != 3 or len(si) not in (1, 2):
+        raise RuntimeError(f"moe_experts: x {tuple(sx)}, w1 {tuple(s1)}, indices {tuple(si)}: need [T, d], [E, d, h], [T, k]")
+    (T, d), (E, d1, h), k = sx, s1, si[-1]
+    if d1 != d or w3.shape != s1 or w2.shape != (E, h, d):
+        raise RuntimeError(f"moe_experts: w1 {tuple(s1)}, w3 {tuple(w3.shape)} must be [E, {d}, h], w2 {tuple(w2.shape)} [E, h, {d}]")
+    if (si != (T, k) and (T != 1 or len(si) != 1)) or indices.dtype not in _WHOLE:
+        raise RuntimeError(f"moe_experts: indices {tuple(si)} {indices.dtype}: need whole numbers, k for each of {T} tokens")
+    bf = torch.bfloat16
+    if not (x.dtype is bf and w1.dtype is bf and w2.dtype is bf and w3.dtype is bf):
         raise RuntimeError("moe_experts: x, w1, w2 and w3 must be bf16")
-    if any(t.device != x.device for t in (w1, w2, w3)):
+    device = x.device
+    if not (w1.device == device and w2.device == device and w3.device == device):
         raise RuntimeError("moe_experts: w1, w2 and w3 must be on the device of x")
-    if weights.shape != (T, k) or weights.device != x.device:
-        weights = weights.to(x.device).expand(T, k)
-    return weights, indices.to(x.device).reshape(T, k)
+    if weights.shape != (T, k) or weights.device != device:
+        weights = weights.to(device).expand(T, k)
+    if len(si) != 2 or indices.device != device:
+        indices = indices.to(device).reshape(T, k)
+    return weights, indices
 
 
 def moe_experts(x: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, w3: torch.Tensor, weights: torch.Tensor, indices: torch.Tensor) -> torch.Tensor:
@@ -293,6 +300,6 @@ def moe_experts(x: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, w3: torch.T
     weights, indices = _expert_operands(x, w1, w2, w3, weights, indices)
     if not x.is_cuda:
         raise RuntimeError("moe_experts: x must be on a CUDA device")
-    T, k = indices.shape
-    native = T > 0 and 0 < k <= 8 and w1.shape[1] % 64 == 0 and w1.shape[2] % 64 == 0
+    (T, k), (_, d, h) = indices.shape, w1.shape
+    native = T > 0 and 0 < k <= 8 and d % 64 == 0 and h % 64 == 0
     return (_MoEExpertsFn if native else _MoEExpertsStagedFn).apply(x.contiguous(), w1, w2, w3, weights, indices)

@@ -6,10 +6,10 @@
 // and the tokens its eight columns. A 4-bit value becomes bf16 by a shift and one logic operation ((q << 3) | 0x4180 is 16 + q
 // exactly), the products of a 32-weight group are summed unscaled, and scale and offset enter once per group in fp32:
 //   y += (d s) * sum (16 + q) x  -  (16 d s + dmin m) * sum x
-// The two parts of a group carry 16 sum x, which cancels in fp32: against sums over decoded weights that is at most a few more roundings of 16 times
-// the offset's size (the error against 64 bits is the output's rounding to bf16 in both kernels, 1.66e-3). Where an activation is
-// infinite, undefined or beyond 2^65 the parts would cancel to nothing or overflow, so a token with such a value in a warp's part of K gets that part
-// summed over decoded weights, one by one.
+// The two parts of a group carry 16 sum x, which cancels in fp32: some 2^-20 d s |x| beside a sum over decoded weights, lost in the output's
+// rounding to bf16 for activations of one magnitude (error against 64 bits 1.66e-3 in both kernels). An activation far above the others shows where its
+// weight is nearly zero, an infinite or undefined one gives nothing but NaN. So a token with a value of 2^16 or more (beyond fp16, which such
+// models are run in) in a warp's part of K gets that part summed over decoded weights, one by one.
 // The contraction index is permuted so that a lane's 8 bytes of a group are its operands as they lie; the tokens are put into
 // that order in shared memory once per CTA, with the sums of their groups.
 //
@@ -120,12 +120,11 @@ __device__ __forceinline__ void q4_multiply(const Q4Block& v, const uint4* xs, c
   chunk(integral_constant<int, 6>{}, integral_constant<int, 7>{}, v.q[0][3], v.q[1][3]);
 }
 
-// The larger magnitudes of two pairs (undefined if one is), and whether either value is infinite, undefined or at least 2^65: an exponent field
-// of 192 and above
+// The larger magnitudes of two pairs (undefined if one is), and whether either is 65536 or more, infinite or undefined
 __device__ __forceinline__ __nv_bfloat162 q4_top(__nv_bfloat162 a, uint32_t w) { return __hmax2_nan(a, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w))); }
 __device__ __forceinline__ bool q4_beyond(__nv_bfloat162 a) {
   const uint32_t w = *reinterpret_cast<const uint32_t*>(&a);
-  return w & (w << 1) & 0x40004000u;
+  return (w & 0xFFFFu) >= 0x4780u || (w >> 16) >= 0x4780u;
 }
 
 // sum over blocks k_lo .. k_hi - 1 of one weight row times one token, weight by weight. A call of its own: the kernel has no registers to

@@ -310,7 +310,7 @@ def test_q4k_gemv_of_infinities_and_huge_values(B, N, K):
     w = torch.from_numpy(kquant.dequantize(t, raw.tobytes())).view(N, K).to(dev)
     packed, clean = torch.from_numpy(raw).to(dev).reshape(-1), torch.randn(B, K, device=dev).bfloat16()
     before = infer.kquant_gemv(t, packed, clean, N)
-    for row, col, v in ((0, 0, math.inf), (B - 1, K - 1, -math.inf), (B // 2, K // 2 + 3, math.nan), (0, 37, 2.0 ** 120), (B - 1, 100, -2.0 ** 66)):
+    for row, col, v in ((0, 0, math.inf), (B - 1, K - 1, -math.inf), (B // 2, K // 2 + 3, math.nan), (0, 37, 2.0 ** 120), (B - 1, 100, -2.0 ** 40), (0, 200, 2.0 ** 16)):
         x = clean.clone()
         x[row, col] = v
         got = infer.kquant_gemv(t, packed, x, N).float()
